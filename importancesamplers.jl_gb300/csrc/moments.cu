@@ -1,14 +1,12 @@
 // moments.cu — weighted mean / covariance of the retained samples and the
 // FP64 candidate fit (ridge, Cholesky, Student-t scaling, lognormalizer).
 //
-// weighted_moments is a literal two-pass restatement of _weighted_moments!
+// weighted_moments is a two-pass restatement of _weighted_moments!
 // (src/adaptive_gaussian_execution.jl:268-273): pass 1 the weighted mean about
 // `shift`, pass 2 the weighted covariance about that mean. Weights are
-// w_i = exp(l_i - max) / S from the device summary words. Each block stages a
-// tile of samples in shared memory (centred, in the sample dtype) and
-// accumulates its share of the d or d x d sums; per-block partials are summed
-// in FP64 by a second kernel. fit_factor runs in one CTA with the covariance
-// in shared memory (d <= 64).
+// w_i = exp(l_i - max) / S from the device summary words. Sums run in the data
+// type within a thread and in FP64 across blocks. fit_factor runs in one CTA
+// with the covariance in shared memory (d <= 64).
 #include "issm_device.cuh"
 #include "issm_internal.h"
 #include "trinv.cuh"
@@ -16,130 +14,264 @@
 namespace issm {
 
 constexpr int kMomThreads = 256;
-constexpr int kMomTile = 64;
+constexpr int kCovThreads = 320;  // most threads of a covariance CTA
+constexpr int kMomTile = 64;      // samples staged per step of the covariance pass
 
+// CTAs of either pass: 128 samples each (two staged tiles) until every SM has
+// two. With 2048 samples per CTA a 10,000-sample round ran on 5 of 152 SMs.
 static int moment_blocks(int64_t n) {
-    int64_t b = (n + 2047) / 2048;
+    int64_t b = (n + 127) / 128;
     if (b > kSMs * 2) b = kSMs * 2;
     return b < 1 ? 1 : (int)b;
 }
 
-size_t moments_workspace_bytes(int64_t n, int d) {
-    return sizeof(double) * ((size_t)moment_blocks(n) * (size_t)d * (size_t)d + (size_t)d * (size_t)d + 2 * (size_t)d + 16);
+// Register tile of the covariance pass: R x R entries per thread over the
+// lower triangle of ceil(d / R) x ceil(d / R) tiles. FP32 takes 8 x 8 above
+// d = 16 (64 FMAs per four 16-byte shared loads); smaller d would spend most of an 8 x 8
+// tile on padding. FP64 runs at 1.7 FMAs per clock and SM here, whatever the
+// loads, so it takes the tile with the least padding.
+static int cov_tile(int d, int dtype) { return dtype == ISSM_F32 && d > 16 ? 8 : 4; }
+static int cov_tiles(int d, int R) {
+    const int nb = (d + R - 1) / R;
+    return nb * (nb + 1) / 2;
 }
 
-// pass: 0 -> partial[b][c] = sum w (x_c - shift_c); 1 -> partial[b][r + c d] = sum w z_r z_c
+size_t moments_workspace_bytes(int64_t n, int d) {
+    const int e4 = cov_tiles(d, 4) * 16, e8 = cov_tiles(d, 8) * 64;
+    return sizeof(double) * (size_t)moment_blocks(n) * (size_t)(e4 > e8 ? e4 : e8);
+}
+
+// Rows lo .. hi - 1 of this CTA: whole tiles of 64, contiguous.
+__device__ __forceinline__ void moment_rows(int64_t n, int64_t &lo, int64_t &hi) {
+    const int64_t per = ((n + gridDim.x - 1) / gridDim.x + kMomTile - 1) / kMomTile * kMomTile;
+    lo = min(n, (int64_t)blockIdx.x * per);
+    hi = min(n, lo + per);
+}
+
+// Pass 1: partial[b][c] = sum of w (x_c - c0), c0 the centre rounded to T (the
+// finish adds the same rounded value back). Thread t owns coordinate t mod d of
+// every (256 / d)-th row, so a warp reads consecutive elements. One read of the
+// samples; bound by HBM for FP32 (FP64: a subtraction and an FMA per element).
 template <typename T>
-__global__ void __launch_bounds__(kMomThreads) moments_partial_kernel(const T *__restrict__ x, int d, int64_t n,
-                                                                      const T *__restrict__ lw,
-                                                                      const double *__restrict__ summary,
-                                                                      const double *__restrict__ center, int pass,
-                                                                      double *__restrict__ partial) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *tile = reinterpret_cast<T *>(smem_raw);               // kMomTile x d (centred)
-    T *wt = tile + (size_t)kMomTile * d;                      // kMomTile weights
+__global__ void __launch_bounds__(kMomThreads) mean_partial_kernel(const T *__restrict__ x, int d, int64_t n,
+                                                                   const T *__restrict__ lw,
+                                                                   const double *__restrict__ summary,
+                                                                   const double *__restrict__ center,
+                                                                   double *__restrict__ partial) {
+    __shared__ T wt[kMomThreads];
+    __shared__ double red[kMomThreads];
     const T m = (T)summary[0];
     const T inv = (T)(1.0 / summary[1]);
-    const int entries = pass == 0 ? d : d * d;
-    // each thread owns up to 16 entries of the output
-    T acc[16];
+    const int tid = threadIdx.x, R = kMomThreads / d, c = tid % d, r0 = tid / d;
+    const bool own = r0 < R;
+    const T c0 = (T)center[c];
+    T acc = T(0);
+    int64_t lo, hi;
+    moment_rows(n, lo, hi);
+    for (int64_t t0 = lo; t0 < hi; t0 += kMomThreads) {
+        const int cnt = (int)min((int64_t)kMomThreads, hi - t0);
+        __syncthreads();
+        if (tid < cnt) wt[tid] = dexp(lw[t0 + tid] - m) * inv;
+        __syncthreads();
+        if (own) {
+            const T *xp = x + t0 * d + c;
+#pragma unroll 8
+            for (int r = r0; r < cnt; r += R) acc += wt[r] * (xp[r * d] - c0);
+        }
+    }
+    red[tid] = own ? (double)acc : 0.0;
+    __syncthreads();
+    if (tid < d) {
+        double s = 0.0;
+        for (int r = 0; r < R; ++r) s += red[r * d + tid];
+        partial[(size_t)blockIdx.x * d + tid] = s;
+    }
+}
+
+// Pass 2: sums of w z z^T, z = x - (mean rounded to T), over the lower
+// triangle. A CTA stages 64 samples at a time (coalesced, one rounding per
+// element); thread (h, tile, g) holds one R x R register tile and takes every
+// (H G)-th staged sample, so the eight lanes of a 16-byte shared-load phase read
+// eight rows of an odd number of 16-byte groups (no bank conflicts). Bound by
+// FMA issue with shared-memory operands (FP32) or the FP64 pipe. Single
+// entries of the full square per thread (two shared loads per FMA) on few CTAs
+// took 3.36 ms over the passes of an 8-round FP32 run of 80,056 samples,
+// d = 33, against 0.16 ms; FP64 at n = 100,003, d = 20: 0.72 ms against 0.08.
+template <typename T, int R>
+__global__ void __launch_bounds__(kCovThreads, 2) cov_partial_kernel(const T *__restrict__ x, int d, int64_t n,
+                                                                     const T *__restrict__ lw,
+                                                                     const double *__restrict__ summary,
+                                                                     const double *__restrict__ mean, int tiles, int G,
+                                                                     int H, int LD, double *__restrict__ partial) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *z = reinterpret_cast<T *>(smem_raw);   // kMomTile x LD, columns beyond d zero
+    T *wt = z + (size_t)kMomTile * LD;        // kMomTile weights
+    T *ctr = wt + kMomTile;                   // d
+    const int tid = threadIdx.x, B = blockDim.x;
+    const T m = (T)summary[0];
+    const T inv = (T)(1.0 / summary[1]);
+    for (int c = tid; c < d; c += B) ctr[c] = (T)mean[c];
+    for (int e = tid; e < kMomTile * LD; e += B) z[e] = T(0);
+    const int g = tid % G, unit = tid / G, tile = unit % tiles, h = unit / tiles;
+    int br = 0;
+    while ((br + 1) * (br + 2) / 2 <= tile) ++br;
+    const int bc = tile - br * (br + 1) / 2;
+    T acc[R][R];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] = T(0);
-    const int64_t per_block = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t lo = (int64_t)blockIdx.x * per_block;
-    const int64_t hi = min(n, lo + per_block);
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) acc[i][j] = T(0);
+    const int dq = B / d, dr = B - dq * d;  // (row, column) step of B elements
+    int64_t lo, hi;
+    moment_rows(n, lo, hi);
     for (int64_t t0 = lo; t0 < hi; t0 += kMomTile) {
         const int cnt = (int)min((int64_t)kMomTile, hi - t0);
         __syncthreads();
-        for (int e = threadIdx.x; e < cnt * d; e += blockDim.x) {
-            const int s = e / d, c = e - s * d;
-            tile[e] = (T)((double)x[(t0 + s) * d + c] - center[c]);
-        }
-        for (int s = threadIdx.x; s < cnt; s += blockDim.x) {
-            const T w = dexp(lw[t0 + s] - m) * inv;
-            wt[s] = (pass == 1) ? w : w;
-        }
-        __syncthreads();
+        const T *xp = x + t0 * d;
+        int s = tid / d, c = tid - s * d;
+        for (int e = tid; e < cnt * d;) {
+            T v[4];
+            int at[4];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int e = threadIdx.x + j * kMomThreads;
-            if (e < entries) {
-                T a = acc[j];
-                if (pass == 0) {
-                    for (int s = 0; s < cnt; ++s) a += wt[s] * tile[s * d + e];
-                } else {
-                    const int r = e % d, c = e / d;
-                    for (int s = 0; s < cnt; ++s) a += wt[s] * tile[s * d + r] * tile[s * d + c];
+            for (int u = 0; u < 4; ++u) {  // four loads in flight
+                at[u] = e < cnt * d ? s * LD + c : -1;
+                v[u] = at[u] >= 0 ? xp[e] - ctr[c] : T(0);
+                e += B;
+                s += dq;
+                c += dr;
+                if (c >= d) {
+                    c -= d;
+                    ++s;
                 }
-                acc[j] = a;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (at[u] >= 0) z[at[u]] = v[u];
+        }
+        for (int r = tid; r < cnt; r += B) wt[r] = dexp(lw[t0 + r] - m) * inv;
+        __syncthreads();
+        for (int q = h < H ? h * G + g : cnt; q < cnt; q += H * G) {
+            const T w = wt[q];
+            T a[R], b[R];
+            constexpr int V = 16 / sizeof(T);
+#pragma unroll
+            for (int i = 0; i < R; i += V) {
+                *reinterpret_cast<uint4 *>(a + i) = *reinterpret_cast<const uint4 *>(z + q * LD + br * R + i);
+                *reinterpret_cast<uint4 *>(b + i) = *reinterpret_cast<const uint4 *>(z + q * LD + bc * R + i);
+            }
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const T wa = w * a[i];
+#pragma unroll
+                for (int j = 0; j < R; ++j) acc[i][j] += wa * b[j];
             }
         }
     }
+    // the G sample lanes of a tile (adjacent lanes of one warp), then the H groups in order
+    const int entries = tiles * R * R;
+    double *red = reinterpret_cast<double *>(smem_raw);
+    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const int e = threadIdx.x + j * kMomThreads;
-        if (e < entries) partial[(size_t)blockIdx.x * entries + e] = (double)acc[j];
-    }
-}
-
-// Sum block partials in FP64. pass 0: mean = center + S1 (weights sum to one);
-// pass 1: cov = S2 - s1 s1^T where s1 = sum w (x - mean) (nearly zero).
-__global__ void moments_finish_kernel(const double *__restrict__ partial, int blocks, int d, int pass,
-                                      const double *__restrict__ center, double *__restrict__ out,
-                                      const double *__restrict__ s1) {
-    const int entries = pass == 0 ? d : d * d;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < entries; e += gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int b = 0; b < blocks; ++b) acc += partial[(size_t)b * entries + e];
-        if (pass == 0) {
-            out[e] = center[e] + acc;
-        } else {
-            const int r = e % d, c = e / d;
-            out[e] = acc - (s1 ? s1[r] * s1[c] : 0.0);
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            T v = acc[i][j];
+            for (int off = G >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (g == 0 && h < H) red[h * entries + tile * (R * R) + i * R + j] = (double)v;
         }
+    __syncthreads();
+    for (int e = tid; e < entries; e += B) {
+        double s = red[e];
+        for (int k = 1; k < H; ++k) s += red[k * entries + e];
+        partial[(size_t)blockIdx.x * entries + e] = s;
     }
 }
 
-// residual mean about the pass-1 mean, to correct pass 2
-__global__ void moments_residual_kernel(const double *__restrict__ partial, int blocks, int d,
-                                        double *__restrict__ s1) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < d; e += gridDim.x * blockDim.x) {
-        double acc = 0.0;
-        for (int b = 0; b < blocks; ++b) acc += partial[(size_t)b * d + e];
-        s1[e] = acc;
-    }
+// Block partials summed in FP64: 8 lanes per entry, then in lane order.
+constexpr int kFinLanes = 8;
+__device__ __forceinline__ double finish_sum(const double *__restrict__ partial, int blocks, int entries, int e,
+                                             double (*red)[33]) {
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    double acc = 0.0;
+    if (e < entries)
+        for (int b = ty; b < blocks; b += kFinLanes) acc += partial[(size_t)b * entries + e];
+    red[ty][tx] = acc;
+    __syncthreads();
+    if (ty == 0)
+        for (int r = 1; r < kFinLanes; ++r) acc += red[r][tx];
+    return acc;
 }
 
+// mean = c0 + S1 (the weights sum to one), c0 the centre as the pass rounded it
 template <typename T>
+__global__ void __launch_bounds__(32 * kFinLanes) mean_finish_kernel(const double *__restrict__ partial, int blocks,
+                                                                     int d, const double *__restrict__ center,
+                                                                     double *__restrict__ mean) {
+    __shared__ double red[kFinLanes][33];
+    const int e = blockIdx.x * 32 + (threadIdx.x & 31);
+    const double s = finish_sum(partial, blocks, d, e, red);
+    if (threadIdx.x < 32 && e < d) mean[e] = (double)(T)center[e] + s;
+}
+
+// cov = S2 - delta delta^T with delta = mean - (mean rounded to T), what the
+// pass's centre differs from the mean by (zero in FP64)
+template <typename T>
+__global__ void __launch_bounds__(32 * kFinLanes) cov_finish_kernel(const double *__restrict__ partial, int blocks,
+                                                                    int d, int R, int tiles,
+                                                                    const double *__restrict__ mean,
+                                                                    double *__restrict__ cov) {
+    __shared__ double red[kFinLanes][33];
+    const int entries = tiles * R * R, e = blockIdx.x * 32 + (threadIdx.x & 31);
+    const double s = finish_sum(partial, blocks, entries, e, red);
+    if (threadIdx.x >= 32 || e >= entries) return;
+    const int tile = e / (R * R), i = e / R % R, j = e % R;
+    int br = 0;
+    while ((br + 1) * (br + 2) / 2 <= tile) ++br;
+    const int r = br * R + i, c = (tile - br * (br + 1) / 2) * R + j;
+    if (r >= d || c > r) return;
+    const double v = s - (mean[r] - (double)(T)mean[r]) * (mean[c] - (double)(T)mean[c]);
+    cov[r + (size_t)c * d] = v;
+    cov[c + (size_t)r * d] = v;
+}
+
+template <typename T, int R>
 static int moments_t(const T *x, int d, int64_t n, const T *lw, const double *summary, const double *shift,
-                     double *mean, double *cov, double *ws, cudaStream_t stream) {
-    const int blocks = moment_blocks(n);
-    double *partial = ws;
-    double *s1 = ws + (size_t)blocks * d * d;
-    const size_t smem = sizeof(T) * ((size_t)kMomTile * d + kMomTile);
-    if (d * d > 16 * kMomThreads) return ISSM_E_UNSUPPORTED;
-    auto kern = moments_partial_kernel<T>;
-    if (smem > 48 * 1024) {
-        const int e = allow_dynamic_smem((const void *)kern);
-        if (e) return e;
-    }
-    { kern<<<blocks, kMomThreads, smem, stream>>>(x, d, n, lw, summary, shift, 0, partial); note_launch(); }
-    { moments_finish_kernel<<<1, 256, 0, stream>>>(partial, blocks, d, 0, shift, mean, nullptr); note_launch(); }
-    { kern<<<blocks, kMomThreads, smem, stream>>>(x, d, n, lw, summary, mean, 1, partial); note_launch(); }
-    { moments_finish_kernel<<<(d * d + 255) / 256, 256, 0, stream>>>(partial, blocks, d, 1, mean, cov, nullptr); note_launch(); }
-    (void)s1;
+                     double *mean, double *cov, double *partial, cudaStream_t stream) {
+    const int blocks = moment_blocks(n), tiles = cov_tiles(d, R);
+    int G = 32;
+    while (G > 1 && tiles * G > kCovThreads) G >>= 1;
+    const int H = max(1, kCovThreads / (tiles * G));  // > 1 for few tiles only (d <= 8)
+    const int threads = (H * tiles * G + 31) / 32 * 32;
+    constexpr int V = 16 / sizeof(T);
+    int LD = (d + R - 1) / R * R;
+    if (LD / V % 2 == 0) LD += V;  // an odd number of 16-byte groups per row
+    const size_t smem = max(sizeof(T) * ((size_t)kMomTile * LD + kMomTile + d),
+                            sizeof(double) * (size_t)H * tiles * R * R);
+    mean_partial_kernel<T><<<blocks, kMomThreads, 0, stream>>>(x, d, n, lw, summary, shift, partial);
+    note_launch();
+    mean_finish_kernel<T><<<(d + 31) / 32, 32 * kFinLanes, 0, stream>>>(partial, blocks, d, shift, mean);
+    note_launch();
+    cov_partial_kernel<T, R><<<blocks, threads, smem, stream>>>(x, d, n, lw, summary, mean, tiles, G, H, LD, partial);
+    note_launch();
+    cov_finish_kernel<T><<<(tiles * R * R + 31) / 32, 32 * kFinLanes, 0, stream>>>(partial, blocks, d, R, tiles, mean,
+                                                                                   cov);
+    note_launch();
     return (int)cudaGetLastError();
 }
 
 int weighted_moments(const void *x, int d, int64_t n, const void *lw, int dtype, const double *summary,
                      const double *shift, double *mean, double *cov, void *ws, size_t ws_bytes,
                      cudaStream_t stream) {
+    if (d > 64) return ISSM_E_UNSUPPORTED;
     if (ws_bytes < moments_workspace_bytes(n, d)) return ISSM_E_WORKSPACE;
-    if (dtype == ISSM_F32)
-        return moments_t<float>((const float *)x, d, n, (const float *)lw, summary, shift, mean, cov, (double *)ws,
-                                stream);
-    return moments_t<double>((const double *)x, d, n, (const double *)lw, summary, shift, mean, cov, (double *)ws,
-                             stream);
+    double *partial = (double *)ws;
+    if (dtype == ISSM_F64)
+        return moments_t<double, 4>((const double *)x, d, n, (const double *)lw, summary, shift, mean, cov, partial,
+                                    stream);
+    if (cov_tile(d, dtype) == 8)
+        return moments_t<float, 8>((const float *)x, d, n, (const float *)lw, summary, shift, mean, cov, partial,
+                                   stream);
+    return moments_t<float, 4>((const float *)x, d, n, (const float *)lw, summary, shift, mean, cov, partial, stream);
 }
 
 // ---- candidate fit ---------------------------------------------------------------
