@@ -72,6 +72,9 @@ template <> __device__ __forceinline__ double qnan<double>() { return __longlong
 
 // Online log-sum-exp over terms: one exp per term, exact special values
 // (NaN propagates, -Inf terms vanish, equal infinities collapse as logaddexp).
+// FP64 exponentials are dear on this GPU: a term too small to change the sum
+// takes none. s >= 1 once a term is in, so e^-37.5 < 2^-54 rounds away when
+// added to it, and s e^-60 when added to 1 (s counts at most the terms).
 template <typename T> struct LseState {
     T m = -num<T>::inf();
     T s = T(0);
@@ -79,11 +82,27 @@ template <typename T> struct LseState {
     __device__ __forceinline__ void add(T t) {
         if (isnan(t)) {
             nan = true;
-        } else if (t > m) {
-            s = (m == -num<T>::inf()) ? T(1) : s * dexp(m - t) + T(1);
-            m = t;
         } else if (t > -num<T>::inf()) {
-            s += (t == m) ? T(1) : dexp(t - m);
+            const bool up = t > m;
+            const T gap = up ? m - t : t - m;  // <= 0; NaN for equal infinities
+            T e = t == m ? T(1) : T(0);
+            if (sizeof(T) == 4 ? t != m : gap > (up ? T(-60) : T(-37.5)) && t != m) e = dexp(gap);
+            s = up ? s * e + T(1) : s + e;
+            m = up ? t : m;
+        }
+    }
+    // the state of other terms
+    __device__ __forceinline__ void merge(T om, T os, bool onan) {
+        nan |= onan;
+        if (om == -num<T>::inf()) return;
+        if (m == -num<T>::inf()) {
+            m = om;
+            s = os;
+        } else if (om > m) {
+            s = s * dexp(m - om) + os;
+            m = om;
+        } else {
+            s += om == m ? os : os * dexp(om - m);
         }
     }
     __device__ __forceinline__ T value() const {

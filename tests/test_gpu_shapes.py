@@ -37,3 +37,97 @@ def test_native_moments_shapes(issm, orc, cuda, dtype, n, d):
     scale = np.outer(sd, sd) + bound * np.outer(spread, spread) + np.finfo(np.float64).tiny
     assert np.all(np.abs(cov.cpu().numpy() - ec.reshape(d, d)) <= bound * scale)
     assert np.array_equal(cov.cpu().numpy(), cov.cpu().numpy().T)
+
+
+def _factor_bank(issm, orc, rng, d, k, dtype, dev, dof=None):
+    loc = (rng.normal(size=(k, d)) * 0.8).astype(dtype)
+    A = rng.normal(size=(k, d, d))
+    fac = np.linalg.cholesky(A @ A.transpose(0, 2, 1) / d + 0.5 * np.eye(d)).astype(dtype)
+    make = (lambda m, L: issm.FactorGaussian(m, L)) if dof is None else (lambda m, L: issm.FactorStudentT(dtype(dof), m, L))
+    db = issm.pack_proposals([make(m, L) for m, L in zip(loc, fac)], dev)
+    dofs = None if db.dofs is None else db.dofs.double().cpu().numpy()
+    ob = orc.BankView(d, orc.GAUSSIAN if dof is None else orc.STUDENT_T, orc.SCALE_FACTOR,
+                      db.locations.double().cpu().numpy(), db.scales.double().cpu().numpy(),
+                      db.lognormalizers.double().cpu().numpy(), dofs,
+                      None if db.range_risk is None else db.range_risk.cpu().numpy())
+    return db, ob
+
+
+# Forward substitution of a factor with condition number below 100 (floor 0.5)
+# in FP32: d rows of up to d roundings of terms no larger than |L||z|; the
+# bound used by the other FP32 kernels, 2e-5 of max(1, |value|), holds with
+# room at d = 64. FP64: the same count of 1.1e-16 roundings, 1e-12.
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k,dof", [
+    (1, 1, 1, None), (31, 3, 2, 4.0), (33, 4, 5, None), (129, 5, 3, None), (127, 8, 17, 6.0), (300, 9, 40, None),
+    (1000, 12, 7, 3.0), (4097, 16, 64, None), (5000, 17, 9, None), (513, 24, 33, None), (2049, 32, 50, 5.0),
+    (700, 33, 13, None), (257, 48, 9, None), (900, 49, 21, None), (2000, 64, 12, 5.0), (130, 63, 2, None)])
+def test_simt_density_shapes(issm, orc, cuda, dtype, n, d, k, dof):
+    """Full, partial and generating denominators over the thread-group splits,
+    the resident and the chunked bank and every padded dimension."""
+    rng = np.random.default_rng(97 * d + k)
+    db, ob = _factor_bank(issm, orc, rng, d, k, dtype, cuda, dof)
+    x = (1.5 * rng.normal(size=(n, d))).astype(dtype)
+    slots = rng.integers(0, k, size=n).astype(np.int32)
+    tx, ts = torch.tensor(x, device=cuda), torch.tensor(slots, device=cuda)
+    coef = np.log(rng.dirichlet(np.ones(k))).astype(dtype)
+    groups = (1 + np.arange(k) % 3).astype(np.int32)
+    tc, tg = torch.tensor(coef, device=cuda), torch.tensor(groups, device=cuda)
+    tol = 1e-12 if dtype == np.float64 else 2e-5
+    for kind, okind in ((issm.native.DENOM_FULL, orc.DENOM_FULL), (issm.native.DENOM_GENERATING, orc.DENOM_GENERATING),
+                        (issm.native.DENOM_PARTIAL, orc.DENOM_PARTIAL)):
+        den = issm.ops.denominator(kind, tc, groups=tg if kind == issm.native.DENOM_PARTIAL else None)
+        fail = issm.ops.new_failures(cuda)
+        got, gen = issm.ops.mixture_logdensity(db, den, tx, slots=ts, failures=fail, generating=True)
+        exp, egen, _ = orc.mixture_logdensity(ob, x.astype(np.float64).reshape(-1), okind, coef.astype(np.float64),
+                                              slots=slots, group_of_slot=groups)
+        for a, b in ((got, exp), (gen, egen)):
+            assert np.all(np.abs(a.double().cpu().numpy() - b) <= tol * np.maximum(1.0, np.abs(b)))
+        assert int(fail[0].item()) == 0
+
+
+@pytest.mark.parametrize("dtype,d,k", [(np.float32, 3, 4), (np.float32, 16, 64), (np.float32, 24, 9),
+                                       (np.float32, 7, 130)])
+def test_simt_two_samples_per_thread(issm, cuda, dtype, d, k):
+    """The size from which threads own two samples: bitwise the numbers of
+    the same rows evaluated in a small call (the per-pair arithmetic and the
+    component order are the same; below the split size)."""
+    n = 152 * 4 * 4 * 128 + 77
+    rng = np.random.default_rng(d)
+    props = [issm.FactorGaussian((rng.normal(size=d)).astype(dtype),
+                                 (np.eye(d) + np.tril(0.2 * rng.normal(size=(d, d)), -1)).astype(dtype)) for _ in range(k)]
+    db = issm.pack_proposals(props, cuda)
+    x = torch.randn(n, d, device=cuda, dtype=torch.float32, generator=torch.Generator(device=cuda).manual_seed(1))
+    den = issm.ops.denominator(issm.native.DENOM_FULL, torch.zeros(k, device=cuda))
+    big = issm.ops.mixture_logdensity(db, den, x)
+    m = 152 * 4 * 128 + 5  # one sample per thread, components not split
+    for lo in (0, n - m):
+        small = issm.ops.mixture_logdensity(db, den, x[lo:lo + m].contiguous())
+        assert torch.equal(big[lo:lo + m], small)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k,dof", [(100, 3, 2, None), (1000, 10, 24, 5.0), (333, 33, 40, None), (4096, 4, 5, None)])
+def test_simt_round_draws_and_weights(issm, cuda, dtype, n, d, k, dof):
+    """A round's samples equal the separate draw's and its weights the
+    separate density's, bitwise up to the component split's merge order."""
+    from oracle import oracle as orc
+    rng = np.random.default_rng(n + d)
+    db, _ = _factor_bank(issm, orc, rng, d, k, dtype, cuda, dof)
+    tdt = torch.float32 if dtype == np.float32 else torch.float64
+    slots = torch.tensor(rng.integers(0, k, size=n).astype(np.int32), device=cuda)
+    normals = torch.tensor(rng.normal(size=n * d).astype(dtype), device=cuda)
+    rn = torch.tensor(rng.normal(size=n * 8).astype(dtype), device=cuda) if dof else None
+    ru = torch.tensor(rng.random(size=n * 8).astype(dtype), device=cuda) if dof else None
+    rad = dict(radial_normals=rn, rn_stride=8, radial_uniforms=ru, ru_stride=8) if dof else {}
+    coef = torch.full((k,), -float(np.log(k)), dtype=tdt, device=cuda)
+    den = issm.ops.denominator(issm.native.DENOM_FULL, coef)
+    db.proposal_ids = torch.arange(1, k + 1, device=cuda)
+    x, lw, pid = issm.ops.mis_round(db, den, slots, normals, **rad)
+    assert torch.equal(x, issm.ops.draw(db, normals, n, slots=slots, **rad))
+    assert torch.equal(lw, -issm.ops.mixture_logdensity(db, den, x, slots=slots))
+    assert torch.equal(pid, slots.long() + 1)
+    one = issm.ops.draw(db, normals, n, fixed_slot=k - 1, **rad)
+    same = issm.ops.draw(db, normals, n, slots=torch.full((n,), k - 1, dtype=torch.int32, device=cuda), **rad)
+    eps = float(np.finfo(dtype).eps)
+    assert torch.allclose(one, same, rtol=4 * eps, atol=64 * eps)
