@@ -131,3 +131,60 @@ def test_simt_round_draws_and_weights(issm, cuda, dtype, n, d, k, dof):
     same = issm.ops.draw(db, normals, n, slots=torch.full((n,), k - 1, dtype=torch.int32, device=cuda), **rad)
     eps = float(np.finfo(dtype).eps)
     assert torch.allclose(one, same, rtol=4 * eps, atol=64 * eps)
+
+
+# The selected elements are exact; the interpolation fraction divides a
+# difference of cumulative weights (each within n 1e-16 of its sum of at most
+# one) by one sample's weight, at least 1e-3 / n here: below 1e-6 for
+# n <= 3e4, and values are compared where neighbouring values are O(1) apart.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("kind", ["smooth", "equal", "integers", "infinite", "offset", "clusters", "huge"])
+@pytest.mark.parametrize("n,d", [(2, 1), (1023, 5), (1025, 3), (30_000, 4)])
+def test_weighted_quantile_levels(issm, orc, cuda, dtype, kind, n, d):
+    rng = np.random.default_rng(n + d)
+    x = rng.normal(size=(n, d))
+    if kind == "equal":
+        x[:] = 2.5
+    elif kind == "integers":
+        x = np.round(2.0 * x)
+    elif kind == "infinite":
+        x[rng.random((n, d)) < 0.2] = np.inf
+        x[rng.random((n, d)) < 0.2] = -np.inf
+    elif kind == "offset":
+        x = 1.0e6 + 1.0e-3 * x
+    elif kind == "clusters":
+        x = np.where(rng.random((n, d)) < 0.5, 1.0e30, -1.0e-30) * (1.0 + 1.0e-7 * x)
+    elif kind == "huge":
+        x = x * (1.0e300 if dtype == torch.float64 else 1.0e38)
+    lw = rng.uniform(-5.0, 0.0, size=n)
+    tx = torch.tensor(x, device=cuda).to(dtype)
+    tl = torch.tensor(lw, device=cuda).to(dtype)
+    probs = [0.0, 0.05, 0.5, 0.95, 1.0]
+    got = issm.quantile(issm.WeightedSamples(tx, tl), probs).cpu().numpy()
+    w = np.exp(tl.double().cpu().numpy())
+    exp = orc.weighted_quantile(tx.double().cpu().numpy().reshape(-1), d, w / w.sum(), probs)
+    nan = np.isnan(exp)  # an interpolation between opposite infinities
+    assert np.array_equal(np.isnan(got), nan)
+    tol = 1e-6 if dtype == torch.float64 else 2e-6
+    with np.errstate(invalid="ignore"):
+        ok = (got == exp) | (np.abs(got - exp) <= tol * np.maximum(np.abs(exp), np.minimum(1.0, np.abs(x).max())))
+    assert np.all(ok | nan), (got[~(ok | nan)], exp[~(ok | nan)])
+
+
+def test_weighted_quantile_beyond_kept_weights(issm, cuda):
+    """More samples than the workspace keeps weights for: equal to the quantile
+    of the same samples' sorted cumulative weights."""
+    n = (1 << 21) + 13
+    g = torch.Generator(device=cuda).manual_seed(3)
+    x = torch.randn(n, 2, device=cuda, dtype=torch.float64, generator=g)
+    lw = torch.rand(n, device=cuda, dtype=torch.float64, generator=g)
+    got = issm.quantile(issm.WeightedSamples(x, lw), [0.1, 0.5])
+    w = torch.softmax(lw, 0)
+    for c in range(2):
+        v, at = torch.sort(x[:, c])
+        cum = torch.cumsum(w[at], 0)
+        for j, p in enumerate((0.1, 0.5)):
+            thr = p * (cum[-1] - w[at[0]]) + w[at[0]]
+            up = int(torch.searchsorted(cum, thr, right=True))
+            # within the neighbouring samples, whose distance bounds any interpolation fraction's rounding
+            assert float(v[up - 2]) <= float(got[j, c]) <= float(v[up + 1])
