@@ -419,37 +419,41 @@ __device__ T radial_multiplier(T dof, const T *rn, const T *ru, bool has_u, uint
     return T(0);
 }
 
-// x = mu_s + L_s (m n) of one row, in place over its normals, with the packed-
-// bank summation order (_native_proposal_coordinate,
-// src/native_execution.jl:238-264): rows descend in groups of four, so every
-// normal a group needs is still there. c: the staged component, or null (then
-// the bank's global arrays). Returns whether every coordinate is finite.
+// The Student-t radial multiplier of sample i (1 for Gaussians; NaN with the
+// failure recorded when the draws are exhausted).
+template <typename T> __device__ __forceinline__ T draw_multiplier(const MixParams<T> &p, int64_t i, int slot) {
+    if (p.family != ISSM_STUDENT_T) return T(1);
+    uint16_t r;
+    const T m = radial_multiplier(p.dofs[slot], p.rnormals + (size_t)i * p.rn_stride,
+                                  p.runiforms ? p.runiforms + (size_t)i * p.ru_stride : nullptr,
+                                  p.runiforms != nullptr && p.ru_stride > 0, &r);
+    if (!r) return m;
+    record_failure(p.failures, p.index_base + i + 1, 0, r);
+    return qnan<T>();
+}
+
+// x = mu_s + L_s (m n) of one row with the packed-bank summation order
+// (_native_proposal_coordinate, src/native_execution.jl:238-264), for every
+// `step`-th group of four coordinates from group g on, from the top down (so
+// out may be in when step is 1: every normal a group needs is still there). c:
+// the staged component, or null (then the bank's global arrays). Returns
+// whether the coordinates formed are finite.
 template <typename T, int D, bool FACTOR>
-__device__ __forceinline__ bool draw_row(const MixParams<T> &p, int64_t i, int slot, const T *c, T *row) {
+__device__ __forceinline__ bool draw_row(const MixParams<T> &p, int slot, const T *c, T m, int g, int step, const T *in,
+                                         T *out) {
     using Ly = Layout<T, D, FACTOR>;
     const int d = p.d;
-    T m = T(1);
-    if (p.family == ISSM_STUDENT_T) {
-        uint16_t r;
-        m = radial_multiplier(p.dofs[slot], p.rnormals + (size_t)i * p.rn_stride,
-                              p.runiforms ? p.runiforms + (size_t)i * p.ru_stride : nullptr,
-                              p.runiforms != nullptr && p.ru_stride > 0, &r);
-        if (r) {
-            record_failure(p.failures, p.index_base + i + 1, 0, r);
-            m = qnan<T>();
-        }
-    }
     const T *mu = c ? c + Ly::kMu : p.loc + (size_t)slot * d;
     bool valid = true;
     if constexpr (FACTOR) {
         const T *L = p.scales + (size_t)slot * d * d;
-        for (int r0 = (d - 1) & ~3; r0 >= 0; r0 -= 4) {
+        const int top = (d - 1) >> 2;
+        for (int r0 = 4 * (top - (top - g % step + step) % step); r0 >= 0; r0 -= 4 * step) {
             T acc[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j] = r0 + j < d ? mu[r0 + j] : T(0);
-            // columns before the group's diagonal block, then its four columns
             for (int q = 0; q < min(d, r0 + 4); ++q) {
-                const T z = row[q] * m;
+                const T z = in[q] * m;
                 T col[4];
                 if (c) {
                     const T *cq = c + Ly::kBody + Ly::off(q) - (q & ~(Ly::V - 1));
@@ -466,15 +470,15 @@ __device__ __forceinline__ bool draw_row(const MixParams<T> &p, int64_t i, int s
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 if (r0 + j < d) {
-                    row[r0 + j] = acc[j];
+                    out[r0 + j] = acc[j];
                     valid &= (bool)isfinite(acc[j]);
                 }
         }
     } else {
-        for (int r = 0; r < d; ++r) {
+        for (int r = g; r < d; r += step) {
             const T sc = p.scale_kind == ISSM_SCALE_SPHERICAL ? p.scales[slot] : p.scales[(size_t)slot * d + r];
-            const T v = mu[r] + sc * (row[r] * m);
-            row[r] = v;
+            const T v = mu[r] + sc * (in[r] * m);
+            out[r] = v;
             valid &= (bool)isfinite(v);
         }
     }
@@ -536,27 +540,33 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
     T *comps = reinterpret_cast<T *>(smem_raw);
     const int d = p.d, tid = threadIdx.x, KS = p.ksplit, GT = kSimtThreads / KS, TR = GT * S;
     T *tile = comps + (size_t)(p.resident ? 1 : 2) * p.chunk * Ly::kStride;
-    T *merge = tile + (size_t)TR * LX;  // ksplit > 1: per thread and sample (max, sum, generating, flags)
+    T *merge = tile + (size_t)TR * LX;           // ksplit > 1: per thread (max, sum, generating, flags),
+    T *mult = merge + 4 * kSimtThreads;          // per sample the radial multiplier,
+    T *drawn_tile = mult + kSimtThreads;         // and the drawn samples
+    __shared__ int s_bad[kSimtThreads], s_lo, s_hi;
     const int grp = tid / GT, si = tid - grp * GT;
     const int nslots = p.mode == kModeDraw ? 0 : p.last_slot - p.first_slot + 1;
     const int nchunks = nslots > 0 ? (nslots + p.chunk - 1) / p.chunk : 0;
     const int64_t ntiles = (p.n + TR - 1) / TR;
     const int my_tiles = (int)((ntiles - (int64_t)blockIdx.x + gridDim.x - 1) / gridDim.x);
-    const int items = my_tiles * nchunks;
-    auto request = [&](int j) {
-        const int k0 = (j % nchunks) * p.chunk;
-        stage_request<T, D, FACTOR>(comps + (size_t)(p.resident ? 0 : j & 1) * p.chunk * Ly::kStride, p,
-                                    p.first_slot + k0, min(p.chunk, nslots - k0));
+    const bool only_own = p.den_kind == ISSM_DENOM_GENERATING;  // a tile needs its own samples' slots only
+    auto request = [&](int ch, int buf) {
+        const int k0 = ch * p.chunk;
+        stage_request<T, D, FACTOR>(comps + (size_t)buf * p.chunk * Ly::kStride, p, p.first_slot + k0,
+                                    min(p.chunk, nslots - k0));
     };
     // coordinates beyond d are read as zeros
-    for (int e = tid; e < TR * LX; e += kSimtThreads) tile[e] = T(0);
-    if (items > 0) request(0);
-    if (p.resident && items > 0) {
+    for (int e = tid; e < TR * LX; e += kSimtThreads) {
+        tile[e] = T(0);
+        if (KS > 1) drawn_tile[e] = T(0);
+    }
+    if (nslots > 0 && (p.resident || !only_own)) request(0, 0);
+    if (p.resident && nslots > 0) {
         tc::cp_async_wait_all();
         __syncthreads();
         stage_finish<T, D, FACTOR>(comps, d, nslots);
     }
-    int item = 0;
+    int item = 0;  // chunks evaluated so far: the buffer in use alternates
     for (int it = 0; it < my_tiles; ++it) {
         const int64_t row0 = ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * TR;
         const int rows = (int)min((int64_t)TR, p.n - row0);
@@ -572,26 +582,46 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
             ok[s] = i < p.n;
             gen[s] = ok[s] ? (p.slots ? p.slots[i] : p.fixed_slot) : 0;
         }
+        T *xs = tile;
         if (drawn) {
-            if (grp == 0) {
+            if (KS == 1) {
 #pragma unroll
                 for (int s = 0; s < S; ++s)
                     if (ok[s]) {
                         const int64_t i = row0 + si + s * GT;
                         const T *c = p.resident && nslots > 0 ? comps + (size_t)gen[s] * Ly::kStride : nullptr;
-                        if (!draw_row<T, D, FACTOR>(p, i, gen[s], c, tile + (size_t)(si + s * GT) * LX)) {
+                        T *row = tile + (size_t)(si + s * GT) * LX;
+                        if (!draw_row<T, D, FACTOR>(p, gen[s], c, draw_multiplier(p, i, gen[s]), 0, 1, row, row)) {
                             record_failure(p.failures, p.index_base + i + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
                             ok[s] = false;
                         }
                     }
+            } else {
+                // every group draws: the samples' multipliers, then the rows' coordinates, are dealt out
+                const int64_t i = row0 + si;
+                if (ok[0] && si % KS == grp) mult[si] = draw_multiplier(p, i, gen[0]);
+                if (grp == 0) s_bad[si] = 0;
+                __syncthreads();
+                if (ok[0]) {
+                    const T *c = p.resident ? comps + (size_t)gen[0] * Ly::kStride : nullptr;
+                    if (!draw_row<T, D, FACTOR>(p, gen[0], c, mult[si], grp, KS, tile + (size_t)si * LX,
+                                                drawn_tile + (size_t)si * LX))
+                        s_bad[si] = 1;
+                }
+                xs = drawn_tile;
             }
             __syncthreads();
-            if (p.samples_out) move_tile<T, LX, false>(tile, p.samples_out + (size_t)row0 * d, rows, d);
+            if (KS > 1 && ok[0] && s_bad[si]) {
+                ok[0] = false;
+                if (grp == 0)
+                    record_failure(p.failures, p.index_base + row0 + si + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
+            }
+            if (p.samples_out) move_tile<T, LX, false>(xs, p.samples_out + (size_t)row0 * d, rows, d);
             if (p.mode == kModeDraw) continue;
             __syncthreads();  // the slow path reads the stored samples
         }
         T x[S][XREG ? D : 1];
-        const T *xt = tile + (size_t)si * LX;
+        const T *xt = xs + (size_t)si * LX;
         if constexpr (XREG) {
 #pragma unroll
             for (int s = 0; s < S; ++s)
@@ -608,7 +638,26 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
             has_gen[s] = false;
             g_gen[s] = (p.den_kind == ISSM_DENOM_PARTIAL && ok[s]) ? p.group[gen[s]] : 0;
         }
-        for (int ch = 0; ch < nchunks; ++ch, ++item) {
+        int ch0 = 0, ch1 = nchunks - 1;
+        if (only_own && !p.resident) {
+            // the chunks that hold the tile's slots (neighbours for a stratified assignment)
+            if (tid == 0) {
+                s_lo = 0x7fffffff;
+                s_hi = -1;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int s = 0; s < S; ++s)
+                if (ok[s]) {
+                    atomicMin(&s_lo, gen[s]);
+                    atomicMax(&s_hi, gen[s]);
+                }
+            __syncthreads();
+            ch0 = max(0, s_lo - p.first_slot) / p.chunk;
+            ch1 = s_hi < 0 ? ch0 - 1 : min(nchunks - 1, (s_hi - p.first_slot) / p.chunk);
+            if (ch0 <= ch1) request(ch0, item & 1);
+        }
+        for (int ch = ch0; ch <= ch1; ++ch, ++item) {
             const T *buf = comps;
             const int k0 = p.first_slot + ch * p.chunk, count = min(p.chunk, p.last_slot - k0 + 1);
             if (!p.resident) {
@@ -616,7 +665,8 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                 tc::cp_async_wait_all();
                 __syncthreads();  // the chunk has landed and the other buffer is free
                 stage_finish<T, D, FACTOR>(b, d, count);
-                if (item + 1 < items) request(item + 1);
+                if (ch < ch1) request(ch + 1, (item + 1) & 1);
+                else if (!only_own && it + 1 < my_tiles) request(0, (item + 1) & 1);
                 __syncthreads();
                 buf = b;
             }
@@ -948,15 +998,16 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     auto tiles_of = [&](int ks) { return (p.n + kSimtThreads / ks * S - 1) / (kSimtThreads / ks * S); };
     // Components are split over thread groups while there are fewer CTAs than
     // the SMs hold (FP32), or than eight waves of them: FP64 runs at the pipe's
-    // rate from one warp per scheduler on, so finer tiles only even out the last wave.
+    // rate from one warp per scheduler on, so finer tiles only even out the last
+    // wave. A generating-only denominator has one component per sample to split.
     int ks = 1;
-    if (S == 1 && nslots > 1)
+    if (S == 1 && nslots > 1 && p.den_kind != ISSM_DENOM_GENERATING)
         while (ks < 4 && nslots >= 2 * ks && tiles_of(ks) < (int64_t)sms * MINB * (sizeof(T) == 8 ? 8 : 1)) ks *= 2;
     p.ksplit = ks;
     const int64_t tiles = tiles_of(ks);
     const size_t per = (size_t)Ly::kStride * sizeof(T);
-    const size_t fixed = (size_t)(kSimtThreads / ks) * S * (D + 1) * sizeof(T) +
-                         (ks > 1 ? (size_t)kSimtThreads * S * 4 * sizeof(T) : 0);
+    const size_t rows_bytes = (size_t)(kSimtThreads / ks) * S * (D + 1) * sizeof(T);
+    const size_t fixed = rows_bytes + (ks > 1 ? (size_t)kSimtThreads * 5 * sizeof(T) + rows_bytes : 0);
     // the bank's share of shared memory with as many CTAs on an SM as the
     // registers allow, or as there are; one fewer where the bank then stays
     int want = (int)max((int64_t)1, min((int64_t)MINB, (tiles + sms - 1) / sms));
@@ -967,7 +1018,7 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     p.chunk = p.resident ? nslots : max(1, (int)(budget / 2 / per));
     const size_t smem = fixed + (p.resident ? 1 : 2) * (size_t)p.chunk * per;
     auto kern = mixture_simt_kernel<T, D, FACTOR, S, MINB>;
-    if (smem > 48 * 1024) {
+    if (smem > 46 * 1024) {  // the limit without opting in, less the static part
         const int e = allow_dynamic_smem((const void *)kern);
         if (e) return e;
     }
