@@ -59,6 +59,7 @@ template <typename T> struct MixParams {
     int first_slot, last_slot;
     int chunk, resident;   // components staged at a time; whether that is all of them, once per CTA
     int ksplit;            // thread groups of a CTA that share its samples and split the components
+    int prefetch;          // two sample tiles: the next one loads while one is evaluated
 };
 
 // ---- slow path ----------------------------------------------------------
@@ -421,14 +422,15 @@ __device__ T radial_multiplier(T dof, const T *rn, const T *ru, bool has_u, uint
 
 // The Student-t radial multiplier of sample i (1 for Gaussians; NaN with the
 // failure recorded when the draws are exhausted).
-template <typename T> __device__ __forceinline__ T draw_multiplier(const MixParams<T> &p, int64_t i, int slot) {
+template <typename T>
+__device__ __forceinline__ T draw_multiplier(const MixParams<T> &p, int64_t i, int slot, bool record = true) {
     if (p.family != ISSM_STUDENT_T) return T(1);
     uint16_t r;
     const T m = radial_multiplier(p.dofs[slot], p.rnormals + (size_t)i * p.rn_stride,
                                   p.runiforms ? p.runiforms + (size_t)i * p.ru_stride : nullptr,
                                   p.runiforms != nullptr && p.ru_stride > 0, &r);
     if (!r) return m;
-    record_failure(p.failures, p.index_base + i + 1, 0, r);
+    if (record) record_failure(p.failures, p.index_base + i + 1, 0, r);
     return qnan<T>();
 }
 
@@ -452,20 +454,37 @@ __device__ __forceinline__ bool draw_row(const MixParams<T> &p, int slot, const 
             T acc[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j] = r0 + j < d ? mu[r0 + j] : T(0);
-            for (int q = 0; q < min(d, r0 + 4); ++q) {
-                const T z = in[q] * m;
-                T col[4];
-                if (c) {
-                    const T *cq = c + Ly::kBody + Ly::off(q) - (q & ~(Ly::V - 1));
+            // columns before the group's diagonal block, then its (up to four) columns
+            if (c) {
+#pragma unroll 4
+                for (int q = 0; q < r0; ++q) {
+                    const T z = in[q] * m;
+                    T col[4];
+                    const T *cq = c + Ly::kBody + Ly::off(q) - (q & ~(Ly::V - 1)) + r0;
+                    *reinterpret_cast<uint4 *>(col) = *reinterpret_cast<const uint4 *>(cq);
+                    if constexpr (sizeof(T) == 8)
+                        *reinterpret_cast<uint4 *>(col + 2) = *reinterpret_cast<const uint4 *>(cq + 2);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) col[j] = r0 + j >= q && r0 + j < D ? cq[r0 + j] : T(0);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) col[j] = r0 + j >= q && r0 + j < d ? L[(size_t)q * d + r0 + j] : T(0);
+                    for (int j = 0; j < 4; ++j) acc[j] += col[j] * z;
                 }
+            } else {
+                for (int q = 0; q < r0; ++q) {
+                    const T z = in[q] * m;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (q <= r0 + j) acc[j] += col[j] * z;
+                    for (int j = 0; j < 4; ++j)
+                        if (r0 + j < d) acc[j] += L[(size_t)q * d + r0 + j] * z;
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int q = r0 + t;
+                if (q < d) {
+                    const T z = in[q] * m;
+                    const T *cq = c ? c + Ly::kBody + Ly::off(q) - (q & ~(Ly::V - 1)) : L + (size_t)q * d;
+#pragma unroll
+                    for (int j = t; j < 4; ++j)
+                        if (r0 + j < d) acc[j] += cq[r0 + j] * z;
+                }
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -481,6 +500,73 @@ __device__ __forceinline__ bool draw_row(const MixParams<T> &p, int slot, const 
             out[r] = v;
             valid &= (bool)isfinite(v);
         }
+    }
+    return valid;
+}
+
+// One short row (d <= D <= 16) between global memory and registers: a thread's
+// whole row is a sector or two, so a shared tile would add only its barriers.
+template <typename T, int D> __device__ __forceinline__ void load_row(const T *g, int d, bool vec, T (&x)[D]) {
+    constexpr int V = 16 / sizeof(T);
+#pragma unroll
+    for (int r0 = 0; r0 < D; r0 += V) {
+        T v[V];
+#pragma unroll
+        for (int j = 0; j < V; ++j) v[j] = T(0);
+        if (vec && r0 < d) load16(g + r0, v);
+        else
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+                if (r0 + j < d) v[j] = g[r0 + j];
+#pragma unroll
+        for (int j = 0; j < V; ++j) x[r0 + j] = v[j];
+    }
+}
+template <typename T, int D> __device__ __forceinline__ void store_row(T *g, int d, bool vec, const T (&x)[D]) {
+    constexpr int V = 16 / sizeof(T);
+#pragma unroll
+    for (int r0 = 0; r0 < D; r0 += V) {
+        if (vec && r0 < d) *reinterpret_cast<uint4 *>(g + r0) = *reinterpret_cast<const uint4 *>(&x[r0]);
+        else
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+                if (r0 + j < d) g[r0 + j] = x[r0 + j];
+    }
+}
+
+// draw_row in registers: x holds the normals, then the sample
+template <typename T, int D>
+__device__ __forceinline__ bool draw_registers(const MixParams<T> &p, int slot, const T *c, T m, T (&x)[D]) {
+    using Ly = Layout<T, D, true>;
+    constexpr int V = Ly::V;
+    const int d = p.d;
+    const T *mu = c ? c + Ly::kMu : p.loc + (size_t)slot * d;
+    const T *L = p.scales + (size_t)slot * d * d;
+    T y[D];
+#pragma unroll
+    for (int r = 0; r < D; ++r) y[r] = r < d ? mu[r] : T(0);
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+        const T z = x[q] * m;
+#pragma unroll
+        for (int r0 = q & ~(V - 1); r0 < D; r0 += V) {
+            T col[V];
+            if (c) {
+                load16(c + Ly::kBody + Ly::off(q) + r0 - (q & ~(V - 1)), col);
+            } else {
+#pragma unroll
+                for (int j = 0; j < V; ++j) col[j] = q < d && r0 + j >= q && r0 + j < d ? L[q * d + r0 + j] : T(0);
+            }
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+                if (r0 + j >= q) y[r0 + j] += col[j] * z;
+        }
+    }
+    bool valid = true;
+#pragma unroll
+    for (int r = 0; r < D; ++r) {
+        x[r] = y[r];
+        if (r < d) valid &= (bool)isfinite(y[r]);
     }
     return valid;
 }
@@ -517,6 +603,28 @@ __device__ __forceinline__ void move_tile(T *tile, T *g, int rows, int d) {
     }
 }
 
+// the same into the tile with asynchronous copies (one commit group)
+template <typename T, int LX> __device__ __forceinline__ void request_tile(T *tile, const T *g, int rows, int d) {
+    constexpr int kB = kSimtThreads;
+    const int dq = kB / d, dr = kB - dq * d, total = rows * d;
+    int r = threadIdx.x / d, c = threadIdx.x - r * d;
+    for (int e = threadIdx.x; e < total; e += kB) {
+        cp_async_elem(tile + r * LX + c, g + e);
+        r += dq;
+        c += dr;
+        if (c >= d) {
+            c -= d;
+            ++r;
+        }
+    }
+    tc::cp_async_commit();
+}
+
+// rows go between global memory and registers, without a tile
+template <typename T, int D, bool FACTOR> __host__ __device__ constexpr bool simt_direct() {
+    return FACTOR && sizeof(T) == 4 && D <= 16;
+}
+
 // Mixture densities, static-MIS rounds, appends and draws. CTAs of 128 threads
 // walk tiles of samples; the bank is staged in shared memory, whole and once
 // per CTA when it fits (`resident`), else in double-buffered chunks prefetched
@@ -535,12 +643,13 @@ template <typename T, int D, bool FACTOR, int S, int MINB>
 __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixParams<T> p) {
     using Ly = Layout<T, D, FACTOR>;
     constexpr bool XREG = FACTOR && sizeof(T) == 4 && D <= 32;  // beyond, x and v together exceed the registers
+    constexpr bool DIRECT = simt_direct<T, D, FACTOR>();
     constexpr int LX = D + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *comps = reinterpret_cast<T *>(smem_raw);
     const int d = p.d, tid = threadIdx.x, KS = p.ksplit, GT = kSimtThreads / KS, TR = GT * S;
-    T *tile = comps + (size_t)(p.resident ? 1 : 2) * p.chunk * Ly::kStride;
-    T *merge = tile + (size_t)TR * LX;           // ksplit > 1: per thread (max, sum, generating, flags),
+    T *tiles = comps + (size_t)(p.resident ? 1 : 2) * p.chunk * Ly::kStride;
+    T *merge = tiles + (DIRECT ? 0 : (size_t)(p.prefetch ? 2 : 1) * TR * LX);  // ksplit > 1: per thread (max, sum, generating, flags),
     T *mult = merge + 4 * kSimtThreads;          // per sample the radial multiplier,
     T *drawn_tile = mult + kSimtThreads;         // and the drawn samples
     __shared__ int s_bad[kSimtThreads], s_lo, s_hi;
@@ -555,11 +664,25 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
         stage_request<T, D, FACTOR>(comps + (size_t)buf * p.chunk * Ly::kStride, p, p.first_slot + k0,
                                     min(p.chunk, nslots - k0));
     };
+    const bool drawn = p.mode == kModeRound || p.mode == kModeDraw;
+    const T *rows_in = drawn ? p.normals : p.x;
+    auto tile_row = [&](int it) -> int64_t { return ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * TR; };
+    auto request_rows = [&](int it) {
+        const int64_t r0 = tile_row(it);
+        request_tile<T, LX>(tiles + (size_t)(it & 1) * TR * LX, rows_in + (size_t)r0 * d, (int)min((int64_t)TR, p.n - r0), d);
+    };
     // coordinates beyond d are read as zeros
-    for (int e = tid; e < TR * LX; e += kSimtThreads) {
-        tile[e] = T(0);
+    for (int e = DIRECT ? TR * LX : tid; e < TR * LX; e += kSimtThreads) {
+        tiles[e] = T(0);
+        if (p.prefetch) tiles[TR * LX + e] = T(0);
         if (KS > 1) drawn_tile[e] = T(0);
     }
+    if (!DIRECT && p.prefetch) {
+        __syncthreads();
+        request_rows(0);
+    }
+    const bool vec = DIRECT && d % Ly::V == 0 &&
+                     ((reinterpret_cast<uintptr_t>(rows_in) | reinterpret_cast<uintptr_t>(p.samples_out)) & 15) == 0;
     if (nslots > 0 && (p.resident || !only_own)) request(0, 0);
     if (p.resident && nslots > 0) {
         tc::cp_async_wait_all();
@@ -568,12 +691,21 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
     }
     int item = 0;  // chunks evaluated so far: the buffer in use alternates
     for (int it = 0; it < my_tiles; ++it) {
-        const int64_t row0 = ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * TR;
+        const int64_t row0 = tile_row(it);
         const int rows = (int)min((int64_t)TR, p.n - row0);
-        __syncthreads();
-        const bool drawn = p.mode == kModeRound || p.mode == kModeDraw;
-        move_tile<T, LX, true>(tile, const_cast<T *>((drawn ? p.normals : p.x) + (size_t)row0 * d), rows, d);
-        __syncthreads();
+        T *tile = tiles;
+        if (DIRECT) {
+            if (it == 0 || KS > 1) __syncthreads();  // the staged bank; the merge buffer
+        } else if (p.prefetch) {
+            tile += (size_t)(it & 1) * TR * LX;
+            tc::cp_async_wait_all();
+            __syncthreads();
+            if (it + 1 < my_tiles) request_rows(it + 1);
+        } else {
+            __syncthreads();
+            move_tile<T, LX, true>(tile, const_cast<T *>(rows_in + (size_t)row0 * d), rows, d);
+            __syncthreads();
+        }
         bool ok[S];
         int gen[S];
 #pragma unroll
@@ -583,7 +715,25 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
             gen[s] = ok[s] ? (p.slots ? p.slots[i] : p.fixed_slot) : 0;
         }
         T *xs = tile;
-        if (drawn) {
+        T x[S][XREG ? D : 1];
+        if constexpr (DIRECT) {
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const int64_t i = row0 + si + s * GT;
+                load_row<T, D>(rows_in + (size_t)(ok[s] ? i : 0) * d, d, vec, x[s]);
+                if (drawn && ok[s]) {
+                    const T *c = p.resident && nslots > 0 ? comps + (size_t)gen[s] * Ly::kStride : nullptr;
+                    ok[s] = draw_registers<T, D>(p, gen[s], c, draw_multiplier(p, i, gen[s], grp == 0), x[s]);
+                    if (grp == 0) {
+                        if (!ok[s])
+                            record_failure(p.failures, p.index_base + i + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
+                        if (p.samples_out) store_row<T, D>(p.samples_out + (size_t)i * d, d, vec, x[s]);
+                    }
+                }
+            }
+            if (p.mode == kModeDraw) continue;
+            if (drawn && KS > 1) __syncthreads();  // the slow path reads the stored samples
+        } else if (drawn) {
             if (KS == 1) {
 #pragma unroll
                 for (int s = 0; s < S; ++s)
@@ -620,9 +770,8 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
             if (p.mode == kModeDraw) continue;
             __syncthreads();  // the slow path reads the stored samples
         }
-        T x[S][XREG ? D : 1];
         const T *xt = xs + (size_t)si * LX;
-        if constexpr (XREG) {
+        if constexpr (XREG && !DIRECT) {
 #pragma unroll
             for (int s = 0; s < S; ++s)
 #pragma unroll
@@ -996,17 +1145,17 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     const int nslots = p.mode == kModeDraw ? 0 : p.last_slot - p.first_slot + 1;
     const int sms = device_sms();
     auto tiles_of = [&](int ks) { return (p.n + kSimtThreads / ks * S - 1) / (kSimtThreads / ks * S); };
-    // Components are split over thread groups while there are fewer CTAs than
-    // the SMs hold (FP32), or than eight waves of them: FP64 runs at the pipe's
+    // Components are split over thread groups while there are fewer than four
+    // CTAs per SM (FP32), or than eight waves of them: FP64 runs at the pipe's
     // rate from one warp per scheduler on, so finer tiles only even out the last
     // wave. A generating-only denominator has one component per sample to split.
     int ks = 1;
     if (S == 1 && nslots > 1 && p.den_kind != ISSM_DENOM_GENERATING)
-        while (ks < 4 && nslots >= 2 * ks && tiles_of(ks) < (int64_t)sms * MINB * (sizeof(T) == 8 ? 8 : 1)) ks *= 2;
+        while (ks < 4 && nslots >= 2 * ks && tiles_of(ks) < (int64_t)sms * min(MINB, 4) * (sizeof(T) == 8 ? 8 : 1)) ks *= 2;
     p.ksplit = ks;
     const int64_t tiles = tiles_of(ks);
     const size_t per = (size_t)Ly::kStride * sizeof(T);
-    const size_t rows_bytes = (size_t)(kSimtThreads / ks) * S * (D + 1) * sizeof(T);
+    const size_t rows_bytes = simt_direct<T, D, FACTOR>() ? 0 : (size_t)(kSimtThreads / ks) * S * (D + 1) * sizeof(T);
     const size_t fixed = rows_bytes + (ks > 1 ? (size_t)kSimtThreads * 5 * sizeof(T) + rows_bytes : 0);
     // the bank's share of shared memory with as many CTAs on an SM as the
     // registers allow, or as there are; one fewer where the bank then stays
@@ -1015,8 +1164,11 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
         --want;
     const size_t budget = kSimtSmem / want - 1024 - fixed;
     p.resident = nslots * per <= budget;
+    // A second tile where it costs no CTA of the bank's: with few components the
+    // tile's loads are most of a CTA's time.
+    p.prefetch = p.resident && tiles > (int64_t)sms * want && nslots * per + rows_bytes <= budget;
     p.chunk = p.resident ? nslots : max(1, (int)(budget / 2 / per));
-    const size_t smem = fixed + (p.resident ? 1 : 2) * (size_t)p.chunk * per;
+    const size_t smem = fixed + (p.prefetch ? rows_bytes : 0) + (p.resident ? 1 : 2) * (size_t)p.chunk * per;
     auto kern = mixture_simt_kernel<T, D, FACTOR, S, MINB>;
     if (smem > 46 * 1024) {  // the limit without opting in, less the static part
         const int e = allow_dynamic_smem((const void *)kern);
@@ -1037,16 +1189,16 @@ template <typename T> static int dispatch_factor(const MixParams<T> &p, cudaStre
     const int d = p.d;
     if constexpr (sizeof(T) == 4) {
         const bool two = p.n >= (int64_t)device_sms() * 4 * 2 * 2 * kSimtThreads;
-#define ISSM_PAIR(DD, MINB)                                            \
+#define ISSM_PAIR(DD, MIN2, MIN1)                                      \
     if (d <= DD)                                                       \
-        return two ? launch_simt<T, DD, true, 2, MINB>(p, stream)      \
-                   : launch_simt<T, DD, true, 1, 4>(p, stream);
-        ISSM_PAIR(4, 4)
-        ISSM_PAIR(8, 4)
-        ISSM_PAIR(12, 4)
-        ISSM_PAIR(16, 4)
-        ISSM_PAIR(24, 3)
-        ISSM_PAIR(32, 3)
+        return two ? launch_simt<T, DD, true, 2, MIN2>(p, stream)      \
+                   : launch_simt<T, DD, true, 1, MIN1>(p, stream);
+        ISSM_PAIR(4, 6, 8)
+        ISSM_PAIR(8, 5, 6)
+        ISSM_PAIR(12, 5, 6)
+        ISSM_PAIR(16, 4, 5)
+        ISSM_PAIR(24, 3, 4)
+        ISSM_PAIR(32, 3, 4)
 #undef ISSM_PAIR
         if (d <= 40) return launch_simt<T, 40, true, 1, 4>(p, stream);
         if (d <= 48) return launch_simt<T, 48, true, 1, 3>(p, stream);
