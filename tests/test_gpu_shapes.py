@@ -188,3 +188,28 @@ def test_weighted_quantile_beyond_kept_weights(issm, cuda):
             up = int(torch.searchsorted(cum, thr, right=True))
             # within the neighbouring samples, whose distance bounds any interpolation fraction's rounding
             assert float(v[up - 2]) <= float(got[j, c]) <= float(v[up + 1])
+
+
+@pytest.mark.parametrize("kind", ["logistic", "linreg"])
+@pytest.mark.parametrize("form", ["bf16", "tf32", "bf16x1"])
+@pytest.mark.parametrize("d,nobs,n", [(2, 1, 127), (16, 255, 128), (17, 256, 129), (32, 1537, 20_000), (33, 31, 40_000),
+                                      (64, 512, 39_000), (64, 513, 300), (5, 33, 60_001)])
+def test_glm_rows_do_not_depend_on_their_tile(issm, cuda, kind, form, d, nobs, n):
+    """Resident and streamed observation tiles, ragged last tiles of both
+    kinds, several row tiles per CTA: every row of a call equals, bitwise, the
+    same row evaluated in a call of its own few neighbours."""
+    rng = np.random.default_rng(nobs + n)
+    X = rng.normal(size=(nobs, d))
+    beta = rng.normal(size=d) / np.sqrt(d)
+    y = (rng.random(nobs) < 0.4).astype(np.float64) if kind == "logistic" else X @ beta + rng.normal(size=nobs)
+    t = issm.LogisticRegressionTarget(X, y, 10.0) if kind == "logistic" else issm.LinearRegressionTarget(X, y, 0.5, 2.0)
+    prec = {"bf16": issm.native.PREC_BF16, "tf32": issm.native.PREC_TF32, "bf16x1": issm.native.PREC_BF16X1}[form]
+    bound = t.bind(cuda, torch.float32)
+    x = torch.tensor((beta + 0.3 * rng.normal(size=(n, d))).astype(np.float32), device=cuda)
+    got = bound.evaluate(x, precision=prec)
+    assert bool(torch.isfinite(got).all())
+    for lo in (0, n // 2 - 50, n - 101, n - 1):
+        lo = max(lo, 0)
+        rows = x[lo:lo + 101].clone()
+        assert torch.equal(got[lo:lo + 101], bound.evaluate(rows, precision=prec))
+    assert int(issm.native.scoped_workspace(cuda, "glm")[:4].view(torch.int32).item()) == 0
