@@ -213,3 +213,36 @@ def test_glm_rows_do_not_depend_on_their_tile(issm, cuda, kind, form, d, nobs, n
         rows = x[lo:lo + 101].clone()
         assert torch.equal(got[lo:lo + 101], bound.evaluate(rows, precision=prec))
     assert int(issm.native.scoped_workspace(cuda, "glm")[:4].view(torch.int32).item()) == 0
+
+
+# A linear predictor is a chain of d FP roundings of terms |x_c b_c| and each
+# observation adds one more; with u the unit roundoff the log target's error is
+# below (d + 8) u sum_o |dl/deta_o| sum_c |x_oc b_c| + 16 u sum_o |l_o|.
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kind", ["logistic", "linreg"])
+@pytest.mark.parametrize("d,nobs,n", [(1, 1, 1), (5, 63, 33), (33, 65, 500), (64, 1100, 127), (65, 64, 40), (130, 200, 70),
+                                      (12, 50, 10_007), (7, 129, 40_001)])
+def test_simt_regression_shapes(issm, cuda, dtype, kind, d, nobs, n):
+    rng = np.random.default_rng(d + nobs)
+    X = rng.normal(size=(nobs, d)).astype(dtype).astype(np.float64)
+    beta = rng.normal(size=d) / np.sqrt(d)
+    y = (rng.random(nobs) < 0.4).astype(np.float64) if kind == "logistic" else X @ beta + 0.5 * rng.normal(size=nobs)
+    y = y.astype(dtype).astype(np.float64)
+    t = issm.LogisticRegressionTarget(X, y, 10.0) if kind == "logistic" else issm.LinearRegressionTarget(X, y, 0.5, 2.0)
+    B = (beta + 0.3 * rng.normal(size=(n, d))).astype(dtype)
+    tdt = torch.float32 if dtype == np.float32 else torch.float64
+    got = t.bind(cuda, tdt).evaluate(torch.tensor(B, device=cuda)).double().cpu().numpy()
+    B64, pv = B.astype(np.float64), 10.0 if kind == "logistic" else 2.0
+    eta, mag = B64 @ X.T, np.abs(B64) @ np.abs(X.T)
+    if kind == "logistic":
+        term, slope = y * eta - np.logaddexp(0.0, eta), np.ones_like(eta)
+        size = np.abs(y * eta) + np.maximum(eta, 0.0) + 1.0
+    else:
+        r = y - eta
+        term, slope = -0.5 * np.log(2 * np.pi * 0.25) - 2.0 * r * r, 4.0 * np.abs(r) + 1.0
+        size = 2.0 * r * r + 1.0
+    prior = -0.5 * d * np.log(2 * np.pi * pv) - (B64 ** 2).sum(1) / (2 * pv)
+    exp = term.sum(1) + prior
+    u = float(np.finfo(dtype).eps) / 2
+    bound = (d + 8) * u * (slope * mag).sum(1) + 16 * u * (size.sum(1) + d * (1.0 + (B64 ** 2).sum(1)))
+    assert np.all(np.abs(got - exp) <= bound)
