@@ -68,7 +68,6 @@ struct QColumn {  // per coordinate
     double w_first;
     float lo, scale;  // level 0: bucket = (v - lo) scale
     int nan;
-    unsigned done;    // CTAs of the running pass that have added their bins
 };
 struct QProblem {  // per (probability, coordinate)
     unsigned long long ka, kb;  // the interval, inclusive
@@ -77,7 +76,7 @@ struct QProblem {  // per (probability, coordinate)
     unsigned long long first;   // least index holding ka
     unsigned count, found;      // samples in the interval; candidates gathered
     int ready, beyond;          // no more levels; threshold not exceeded (the largest value)
-    unsigned done;
+    unsigned done;              // CTAs of the running level that have added their bins
 };
 struct QCandidates {
     unsigned long long key[kQCand];
@@ -284,7 +283,6 @@ __global__ void __launch_bounds__(kQThreads) quantile_setup_kernel(const T *__re
         col.kmax = kmax;
         col.nan = nan | (none ? 1 : 0);
         col.w_first = none ? 0.0 : qweight((double)lw[imin], m, inv);
-        col.done = 0u;
         const float lo = none ? 0.f : fmaxf((float)QK::value(kmin), -3e38f);
         const float hi = none ? 0.f : fminf((float)QK::value(kmax), 3e38f);
         const float scale = (float)kQBins / (hi - lo);
@@ -376,12 +374,10 @@ __device__ __forceinline__ void q_flush(QBins *dst, const double *w, const unsig
 template <typename T>
 __global__ void __launch_bounds__(kQThreads) quantile_level0_kernel(const T *__restrict__ x, int d, int64_t n,
                                                                     const T *__restrict__ lw,
-                                                                    const double *__restrict__ summary, int nprob,
-                                                                    QWork q) {
+                                                                    const double *__restrict__ summary, QWork q) {
     extern __shared__ __align__(16) unsigned char smem[];
     double *bw = reinterpret_cast<double *>(smem);                        // kQCols x kQBins
     unsigned *bn = reinterpret_cast<unsigned *>(bw + kQCols * kQBins);    // kQCols x kQBins
-    __shared__ bool last;
     const int c0 = blockIdx.y * kQCols, nc = min(kQCols, d - c0);
     for (int b = threadIdx.x; b < kQCols * kQBins; b += kQThreads) {
         bw[b] = 0.0;
@@ -413,41 +409,34 @@ __global__ void __launch_bounds__(kQThreads) quantile_level0_kernel(const T *__r
     }
     __syncthreads();
     for (int j = 0; j < nc; ++j) q_flush(q.bins0 + c0 + j, bw + j * kQBins, bn + j * kQBins);
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&q.col[c0].done, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int j = 0; j < nc; ++j) {
-        const QColumn col = q.col[c0 + j];
-        if (col.nan) continue;
-        for (int p = 0; p < nprob; ++p) {
-            QProblem &s = q.prob[(size_t)p * d + c0 + j];
-            double under;
-            unsigned count;
-            const int b = q_choose(q.bins0 + c0 + j, 0.0, s.thr, &under, &count);
-            if (threadIdx.x < 32) {
-                if (b == kQBins) {
-                    if (threadIdx.x == 0) {
-                        s.beyond = 1;  // rounding left the threshold at or above W
-                        s.ready = 1;
-                    }
-                } else {
-                    const unsigned long long ka = q_first_key<T>(col.kmin, col.kmax, b, col.lo, col.scale);
-                    const unsigned long long kz =
-                        b + 1 < kQBins ? q_first_key<T>(ka, col.kmax, b + 1, col.lo, col.scale) : col.kmax + 1;
-                    if (threadIdx.x == 0) {
-                        s.ka = ka;
-                        s.kb = kz - 1;
-                        s.below = under;
-                        s.count = count;
-                        s.ready = count <= (unsigned)kQCand || kz - 1 == ka;
-                    }
-                }
-            }
-            __syncthreads();
+}
+
+// one CTA per problem: the bucket of level 0 and its key interval
+template <typename T> __global__ void __launch_bounds__(kQThreads) quantile_choose0_kernel(int d, QWork q) {
+    const int pr = blockIdx.x;
+    const QColumn col = q.col[pr % d];
+    if (col.nan) return;
+    QProblem &s = q.prob[pr];
+    double under;
+    unsigned count;
+    const int b = q_choose(q.bins0 + pr % d, 0.0, s.thr, &under, &count);
+    if (threadIdx.x >= 32) return;
+    if (b == kQBins) {
+        if (threadIdx.x == 0) {
+            s.beyond = 1;  // rounding left the threshold at or above W
+            s.ready = 1;
         }
+        return;
+    }
+    const unsigned long long ka = q_first_key<T>(col.kmin, col.kmax, b, col.lo, col.scale);
+    const unsigned long long kz =
+        b + 1 < kQBins ? q_first_key<T>(ka, col.kmax, b + 1, col.lo, col.scale) : col.kmax + 1;
+    if (threadIdx.x == 0) {
+        s.ka = ka;
+        s.kb = kz - 1;
+        s.below = under;
+        s.count = count;
+        s.ready = count <= (unsigned)kQCand || kz - 1 == ka;
     }
 }
 
@@ -703,7 +692,9 @@ static int weighted_quantile_t(const T *x, int d, int64_t n, const T *lw, const 
     if (st) return st;
     // row CTAs per column group: two CTAs on every SM, at least 1,024 rows each
     const int rows = (int)max((int64_t)1, min((n + 1023) / 1024, (int64_t)max(1, 2 * sms / cg)));
-    quantile_level0_kernel<T><<<dim3(rows, cg), kQThreads, smem, stream>>>(x, d, n, lw, summary, nprob, q);
+    quantile_level0_kernel<T><<<dim3(rows, cg), kQThreads, smem, stream>>>(x, d, n, lw, summary, q);
+    note_launch();
+    quantile_choose0_kernel<T><<<P, kQThreads, 0, stream>>>(d, q);
     note_launch();
     // each level takes 11 bits of the interval; a problem that is ready returns at once
     const int rows_l = (int)max((int64_t)1, min((n + 4095) / 4096, (int64_t)32));

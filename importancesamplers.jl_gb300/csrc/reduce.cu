@@ -346,8 +346,11 @@ __global__ void __launch_bounds__(256) form_summary_kernel(const T *__restrict__
     summary_finish(ts, out, partials, counter);
 }
 
-static int summary_blocks(int64_t n) {
-    int64_t b = (n + 256 * 16 - 1) / (256 * 16);
+// CTAs of a summary: 16 weights per thread; FP64 weights take an FP64
+// exponential each in a serial chain, so two (57 us at n = 100,003 with 16).
+static int summary_blocks(int64_t n, int dtype) {
+    const int64_t per = 256 * (dtype == ISSM_F32 ? 16 : 2);
+    int64_t b = (n + per - 1) / per;
     if (b > kSMs * 8) b = kSMs * 8;
     return b < 1 ? 1 : (int)b;
 }
@@ -368,7 +371,7 @@ static int summary_launch(const void *lw, int64_t n, int dtype, double *out, voi
     Moments3 *partials = (Moments3 *)((char *)ws + 256);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream);
     if (e != cudaSuccess) return (int)e;
-    const int blocks = summary_blocks(n);
+    const int blocks = summary_blocks(n, dtype);
     if (dtype == ISSM_F32)
         { summary_kernel<float><<<blocks, 256, 0, stream>>>((const float *)lw, n, out, partials, counter); note_launch(); }
     else
@@ -390,7 +393,7 @@ int amis_form_summary(const void *lt, const void *lnum, const int64_t *round_ids
     Moments3 *partials = (Moments3 *)((char *)ws + 256);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream);
     if (e != cudaSuccess) return (int)e;
-    const int blocks = summary_blocks(n);
+    const int blocks = summary_blocks(n, dtype);
     if (dtype == ISSM_F32)
         { form_summary_kernel<float><<<blocks, 256, 0, stream>>>((const float *)lt, (const float *)lnum, round_ids,
                                                                (float)logtotal, n, (float *)lw, failures, out,

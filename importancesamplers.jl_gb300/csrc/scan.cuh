@@ -40,13 +40,19 @@ template <typename A> __device__ A block_exclusive_scan(A v, A *total) {
     return warp_prefix + inc - v;
 }
 
+// keep (may be null): the items as loaded, for a second phase that need not
+// form them again.
 template <typename A, typename Load>
-__global__ void __launch_bounds__(kScanThreads) scan_tile_sums(int64_t n, Load load, A *tile_sums) {
+__global__ void __launch_bounds__(kScanThreads) scan_tile_sums(int64_t n, Load load, A *tile_sums, A *keep) {
     const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     A acc = A(0);
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j)
-        if (base + j < n) acc += load(base + j);
+        if (base + j < n) {
+            const A v = load(base + j);
+            acc += v;
+            if (keep) keep[base + j] = v;
+        }
     A total;
     block_exclusive_scan<A>(acc, &total);
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
@@ -94,9 +100,27 @@ template <typename A, typename Load, typename Write>
 int scan_apply(int64_t n, Load load, Write write, A *ws, cudaStream_t stream) {
     if (n <= 0) return 0;
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    { scan_tile_sums<A, Load><<<(unsigned)tiles, kScanThreads, 0, stream>>>(n, load, ws); note_launch(); }
+    { scan_tile_sums<A, Load><<<(unsigned)tiles, kScanThreads, 0, stream>>>(n, load, ws, nullptr); note_launch(); }
     { scan_tile_prefix<A><<<1, 1024, 0, stream>>>(ws, tiles); note_launch(); }
     { scan_tile_apply<A, Load, Write><<<(unsigned)tiles, kScanThreads, 0, stream>>>(n, load, write, ws, tiles); note_launch(); }
+    return (int)cudaGetLastError();
+}
+
+template <typename A> struct KeptItems {
+    const A *items;
+    __device__ A operator()(int64_t i) const { return items[i]; }
+};
+
+// scan_apply whose items are formed once and kept in `items` (n of A) between
+// the phases: for items that cost more than a read. `write` may overwrite them.
+template <typename A, typename Load, typename Write>
+int scan_apply_kept(int64_t n, Load load, Write write, A *ws, A *items, cudaStream_t stream) {
+    if (n <= 0) return 0;
+    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+    { scan_tile_sums<A, Load><<<(unsigned)tiles, kScanThreads, 0, stream>>>(n, load, ws, items); note_launch(); }
+    { scan_tile_prefix<A><<<1, 1024, 0, stream>>>(ws, tiles); note_launch(); }
+    { scan_tile_apply<A, KeptItems<A>, Write><<<(unsigned)tiles, kScanThreads, 0, stream>>>(n, KeptItems<A>{items}, write,
+                                                                                        ws, tiles); note_launch(); }
     return (int)cudaGetLastError();
 }
 

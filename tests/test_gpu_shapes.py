@@ -246,3 +246,28 @@ def test_simt_regression_shapes(issm, cuda, dtype, kind, d, nobs, n):
     u = float(np.finfo(dtype).eps) / 2
     bound = (d + 8) * u * (slope * mag).sum(1) + 16 * u * (size.sum(1) + d * (1.0 + (B64 ** 2).sum(1)))
     assert np.all(np.abs(got - exp) <= bound)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("d", [1, 2, 3, 4, 6, 33, 64, 130])
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_gather_rows_and_alignments(issm, cuda, dtype, d, offset):
+    n, count = 777, 5003
+    src = torch.randn(n * d + offset, device=cuda, dtype=dtype)[offset:].view(n, d)
+    anc = torch.randint(1, n + 1, (count,), device=cuda)
+    assert torch.equal(issm.ops.gather(src, anc), src[anc - 1])
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 70_001])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_resampling_kept_weights(issm, orc, cuda, n, dtype):
+    """The fixed-point prefix over whole and ragged scan tiles: bit-exact
+    ancestors (the weights formed once and kept)."""
+    rng = np.random.default_rng(n)
+    lw = (rng.normal(size=n) * 2.0).astype(dtype)
+    u = rng.random(size=999)
+    tl = torch.tensor(lw, device=cuda)
+    got = issm.ops.resample_multinomial(tl, torch.tensor(u, device=cuda)).cpu().numpy()
+    assert np.array_equal(got, orc.resample_multinomial_fixed(lw.astype(np.float64), u))
+    got = issm.ops.resample_systematic(tl, 0.37, 500).cpu().numpy()
+    assert np.array_equal(got, orc.resample_systematic_fixed(lw.astype(np.float64), 0.37, 500))
