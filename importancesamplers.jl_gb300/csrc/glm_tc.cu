@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
     __shared__ GlmPair s_bb[4][kGlmRows], s_part[4][kGlmParts - 1][kGlmRows];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tc::uniform_warp(), lane = tid & 31;
     const int R = p.ring, T = p.tiles;
     if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
     if (tid == 0) {
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tbase = tmem_base;
+    const uint32_t tbase = tc::uniform(tmem_base);
     auto wait = [&](uint64_t *bar, uint32_t parity) -> bool {
         if (abort_flag) return false;
         if (tc::mbar_wait(bar, parity)) return true;
@@ -198,13 +198,14 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
         int ok = 1, it = 0, t = 0;
         for (int64_t j = 0; j < J && ok; ++j) {
             const int slot = resident ? t : (int)(j % R);
-            if (lane == 0) {
+            {
                 bool fine = t != 0 || wait(&a_full[it & 1], (uint32_t)((it >> 1) & 1));
                 if (fine && (!resident || it == 0)) {
                     fine = wait(&b_full[slot], resident ? 0u : (uint32_t)((j / R) & 1));
                     if (fine) waited = j + 1;
                 }
                 if (fine && j >= 2) fine = wait(&d_empty[j & 1], (uint32_t)(((j - 2) >> 1) & 1));
+                fine = __all_sync(0xffffffffu, fine);
                 tc::fence_after_sync();
                 if (fine) {
                     const uint32_t dt = tbase + (uint32_t)((j & 1) * kGlmCols);
@@ -215,24 +216,23 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
                         const uint64_t da = tc::smem_desc(a0 + s * 2 * LBO_A, LBO_A, 128);
                         const uint64_t db = tc::smem_desc(b0 + s * 2 * LBO_B, LBO_B, 128);
                         if (KIND == tc::kTF32) {
-                            tc::mma_tf32(dt, da, db, idesc, s > 0);
+                            tc::mma_tf32_elect(dt, da, db, idesc, s > 0);
                         } else {
-                            tc::mma(dt, da, db, idesc, s > 0);
+                            tc::mma_elect(dt, da, db, idesc, s > 0);
                             if (SPLIT == 3) {
                                 const uint64_t dal = tc::smem_desc(a0 + (uint32_t)S::A_PART + s * 2 * LBO_A, LBO_A, 128);
                                 const uint64_t dbl = tc::smem_desc(b0 + (uint32_t)S::B_PART + s * 2 * LBO_B, LBO_B, 128);
-                                tc::mma(dt, dal, db, idesc, true);
-                                tc::mma(dt, da, dbl, idesc, true);
+                                tc::mma_elect(dt, dal, db, idesc, true);
+                                tc::mma_elect(dt, da, dbl, idesc, true);
                             }
                         }
                     }
                 }
-                tc::commit(&d_full[j & 1]);  // arrives when this item's MMAs (issued or not) are done
-                if (!resident) tc::commit(&b_empty[slot]);
-                if (t == T - 1) tc::commit(&a_empty[it & 1]);
+                tc::commit_elect(&d_full[j & 1]);  // arrives when this item's MMAs (issued or not) are done
+                if (!resident) tc::commit_elect(&b_empty[slot]);
+                if (t == T - 1) tc::commit_elect(&a_empty[it & 1]);
                 if (!fine) ok = 0;
             }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
             // refill the slot the previous item's MMAs have finished with
             if (ok && !resident && j >= 1 && j + R - 1 < J) {
                 int fine = 1;

@@ -15,62 +15,32 @@
 //   BF16x3  operands split v = hi + lo in bf16, D = Xh Wh + Xl Wh + Xh Wl,
 //           about 16 significant bits per product.
 //
-// Two kernels per launch:
+// Components that fit one 256-column accumulator (and the shared memory beside
+// the staged tiles) run here; more of them in mixture_pair.cu. Two kernels per
+// launch:
 //   tc_prepare_kernel  one CTA per slot: W_k in MMA operand form (bf16 hi/lo
 //                      or tf32, row-contiguous canonical layout) and b_k;
-//   mixture_tc_kernel  persistent, 8 warps, one 128-sample tile at a time:
-//     * sample tiles stream in with cp.async (16-byte, L1 bypass) into a ring
-//       of padded shared-memory stages, prefetched raw_stages tiles ahead;
-//     * all threads centre, round and split the tile into the A operand
-//       (double-buffered, so converting tile t+1 overlaps MMAs of tile t);
-//     * component operands arrive by bulk copies on an mbarrier, double-
-//       buffered by chunk when a tile needs several chunks of components;
-//     * one thread issues the MMAs of item j (tile, component chunk) into one
-//       of two TMEM accumulators while all warps run the epilogue of item
-//       j-1 from the other: warp w reads TMEM lanes 32 (w mod 4).. and takes
-//       the components of parity w / 4; the two halves merge their
-//       log-sum-exp states through shared memory when the tile completes.
+//   mixture_tc_kernel  persistent, one 128-sample tile at a time:
+//     * warps 1-8 stream sample tiles with cp.async into a ring of padded
+//       stages and centre, round and split each into the A operand (two or
+//       three buffers, so converting tile t+1 overlaps MMAs of tile t);
+//     * warp 0 copies the operands once and issues the MMAs of a tile into one
+//       of two TMEM accumulators;
+//     * warps 9-12 (one per TMEM lane quadrant) run the epilogue of the other.
 // Every wait is bounded; a timeout sets the sticky error word and the CTA
 // unwinds after draining its outstanding copies and MMAs.
-#include "issm_device.cuh"
-#include "issm_internal.h"
-#include "tcgen05.cuh"
+#include "mixture_tc.cuh"
 #include "trinv.cuh"
 
 namespace issm {
 
-constexpr int kTcTile = 128;
-constexpr size_t kTcMaxSmem = 232448 - 1024;  // dynamic shared memory per CTA, static part reserved
-
-__device__ __forceinline__ uint32_t tf32_bits(float f) {
-    uint32_t u = __float_as_uint(f);
-    if ((u & 0x7f800000u) == 0x7f800000u) return u;
-    u += 0xFFFu + ((u >> 13) & 1u);
-    return u & ~0x1FFFu;
-}
-
-// 16 bytes of operand values from v[PER]: 4 tf32 (nearest even), or 8 bf16
-// (the hi part; pack_lo gives the lo part bf16(v - hi)).
-template <int KIND> __device__ __forceinline__ uint4 pack_hi(const float *v) {
-    if (KIND == tc::kTF32) return make_uint4(tc::tf32_rn(v[0]), tc::tf32_rn(v[1]), tc::tf32_rn(v[2]), tc::tf32_rn(v[3]));
-    return make_uint4(tc::pack_bf16x2(v[0], v[1]), tc::pack_bf16x2(v[2], v[3]), tc::pack_bf16x2(v[4], v[5]),
-                      tc::pack_bf16x2(v[6], v[7]));
-}
-__device__ __forceinline__ uint32_t lo_pair(float a, float b, uint32_t hi) {
-    return tc::pack_bf16x2(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
-}
-__device__ __forceinline__ uint4 pack_lo(const float *v, uint4 hi) {
-    return make_uint4(lo_pair(v[0], v[1], hi.x), lo_pair(v[2], v[3], hi.y), lo_pair(v[4], v[5], hi.z),
-                      lo_pair(v[6], v[7], hi.w));
-}
-
 // Operand form of slot k: the DP x (DP + X) matrix [W_k | -b_k | 0], X = 16
 // bf16 or 8 tf32 elements (two extra 16-byte K groups), so the MMA yields
 // z = W_k (x - c) - b_k directly against samples extended by a constant 1.
-// Slots are grouped in chunks of `chunk` consecutive slots; chunk g holds
-// NPART parts of KGX = KG + 2 K groups: part p, K group q, slot kk, row j at
-//   g * NPART*chunk*B + p * chunk*B + q * chunk*DP*16 + kk * DP*16 + j * 16
-// (B = DP*KGX*16), the shared-memory layout of one chunk.
+// The `chunk` slots of a launch are one block of NPART parts of KGX = KG + 2 K
+// groups: part p, K group q, slot kk, row j at
+//   p * chunk*B + q * chunk*DP*16 + kk * DP*16 + j * 16
+// (B = DP*KGX*16), the block's shared-memory layout.
 template <int KIND, int SPLIT, int DP>
 __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict__ w, const float *__restrict__ loc,
                                                          int d, int first, int chunk, int cslot,
@@ -101,10 +71,7 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
         nb[j] = -acc;
     }
     __syncthreads();
-    // chunk-contiguous: the operands of slots first + g*chunk .. are one block
-    // laid out as the MMA reads them (part, K group, slot in chunk, row)
-    const int g = (int)blockIdx.x / chunk, kk = (int)blockIdx.x % chunk;
-    unsigned char *okp = ops + (size_t)g * NPART * chunk * B_COMP + (size_t)kk * DP * 16;
+    unsigned char *okp = ops + (size_t)blockIdx.x * DP * 16;
     for (int e = threadIdx.x; e < KGX * DP; e += blockDim.x) {
         const int q = e / DP, j = e - q * DP;
         float v[PER];
@@ -118,33 +85,18 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
     }
 }
 
-struct TcParams {
-    int d, mode, family, den_kind, fixed_slot;
-    int first_slot, last_slot, chunk, nchunks, ntiles, raw_stages, bring;
-    int64_t n;
-    const float *x;
-    const unsigned char *ops;
-    const float *center;
-    const float *lognorm, *coef, *dofs;
-    const int32_t *group;
-    float *out_logden, *out_generating, *lognum;
-    uint64_t *failures;
-    int64_t index_base;
-    int *error;
-};
-
 // Warp roles of mixture_tc_kernel.
 constexpr int kConvWarps = 8;  // stage sample tiles and build the A operand
 constexpr int kEpiWarps = 4;   // one per TMEM lane quadrant
 constexpr int kConvThreads = 32 * kConvWarps;
 constexpr int kFirstEpiWarp = 1 + kConvWarps;
 constexpr int kTcThreads = 32 * (1 + kConvWarps + kEpiWarps);
-constexpr int kBRing = 3;      // operand buffers in flight when a tile needs several chunks
+constexpr int kRawStages = 3;  // sample tiles staged ahead
 
 // NOB: one component centred at its own location, whose offset column
 // -W (mu - c) is therefore zero: the MMAs run over the coordinates' K groups
 // only (K = DP instead of DP + 16), and three A buffers fit.
-template <int KIND, int SPLIT, int DP, bool DIRECT, bool NOB>
+template <int KIND, int SPLIT, int DP, bool NOB>
 __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
     constexpr int EB = KIND == tc::kBF16 ? 2 : 4;
     constexpr int PER = 16 / EB;              // elements per 16-byte K group
@@ -159,12 +111,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
     constexpr int B_COMP = DP * KGB * 16;
     constexpr int KSTEPS = KGX / 2;           // MMA K slices of 32 bytes
     constexpr uint32_t LBO_A = kTcTile * 16;
-    const int chunk = p.chunk, nchunks = p.nchunks, S = p.raw_stages;
-    // one component chunk: A double-buffered, the chunk's operands loaded once;
-    // several chunks: one A buffer (a tile is converted once per nchunks items)
-    // and a ring of kBRing operand buffers filled kBRing - 1 items ahead
-    const int nbufA = nchunks > 1 ? 1 : NOB ? 3 : 2;
-    const int nbufB = nchunks > 1 ? p.bring : 1;
+    const int chunk = p.nslots;  // components, all in one accumulator
+    constexpr int S = kRawStages, nbufA = NOB ? 3 : 2;
     const uint32_t LBO_B = (uint32_t)(chunk * DP * 16);
     const uint32_t CHUNK_BYTES = (uint32_t)(NPART * chunk * B_COMP);
 
@@ -172,12 +120,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
     unsigned char *s_raw = smem;
     unsigned char *s_a = s_raw + (size_t)S * RAW_BYTES;
     unsigned char *s_b = s_a + (size_t)nbufA * NPART * A_PART;
-    float *s_c = reinterpret_cast<float *>(s_b + (size_t)nbufB * CHUNK_BYTES);
-    __shared__ __align__(8) uint64_t a_full[3], a_empty[3], b_full[kBRing], b_empty[kBRing], d_full[2], d_empty[2];
+    float *s_c = reinterpret_cast<float *>(s_b + CHUNK_BYTES);
+    __shared__ __align__(8) uint64_t a_full[3], a_empty[3], b_full, d_full[2], d_empty[2];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tc::uniform_warp(), lane = tid & 31;
     const int NW = chunk * DP;  // TMEM columns of one accumulator
     const uint32_t ncols = 2 * NW <= 32 ? 32 : 2 * NW <= 64 ? 64 : 2 * NW <= 128 ? 128 : 2 * NW <= 256 ? 256 : 512;
     if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
@@ -190,10 +138,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
             tc::mbar_init(&d_full[b], 1);
             tc::mbar_init(&d_empty[b], kEpiWarps);
         }
-        for (int b = 0; b < kBRing; ++b) {
-            tc::mbar_init(&b_full[b], 1);
-            tc::mbar_init(&b_empty[b], 1);
-        }
+        tc::mbar_init(&b_full, 1);
         tc::fence_mbar_init();
         abort_flag = 0;
     }
@@ -211,15 +156,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tbase = tmem_base;
+    const uint32_t tbase = tc::uniform(tmem_base);
 
     const int my_tiles = (p.ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int J = my_tiles * nchunks;
     auto tile_of = [&](int it) -> int64_t { return (int64_t)blockIdx.x + (int64_t)it * gridDim.x; };
-    auto chunk_range = [&](int ch, int &k0, int &cnt) {
-        k0 = p.first_slot + ch * chunk;
-        cnt = min(chunk, p.last_slot - k0 + 1);
-    };
     // bounded wait that gives up at once after any role has timed out
     auto wait = [&](uint64_t *bar, uint32_t parity) -> bool {
         if (abort_flag) return false;
@@ -231,75 +171,51 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
 
     if (warp == 0) {
         // ================= issuer: component operands and MMAs =================
-        int b_issued = 0, b_waited = 0;
-        // the chunk's operands are one contiguous block in the workspace, laid
-        // out as in shared memory: one bulk copy per item
-        auto issue_b = [&](int j) {
-            const int buf = j % nbufB;
-            if (lane == 0) {
-                tc::mbar_arrive_expect_tx(&b_full[buf], CHUNK_BYTES);
-                tc::bulk_copy_g2s(s_b + (size_t)buf * CHUNK_BYTES, p.ops + (size_t)(j % nchunks) * CHUNK_BYTES,
-                                  CHUNK_BYTES, &b_full[buf]);
-            }
-            __syncwarp();
-            ++b_issued;
-        };
-        // single chunk: its operands once; several: fill the ring
-        for (int q = 0; q < nbufB && q < J; ++q) issue_b(q);
-        for (int j = 0; j < J; ++j) {
-            const int it = j / nchunks, ch = j - it * nchunks;
+        // the operands are one contiguous block in the workspace, laid out as
+        // in shared memory: one bulk copy
+        if (lane == 0 && my_tiles > 0) {
+            tc::mbar_arrive_expect_tx(&b_full, CHUNK_BYTES);
+            tc::bulk_copy_g2s(s_b, p.ops, CHUNK_BYTES, &b_full);
+        }
+        __syncwarp();
+        for (int it = 0; it < my_tiles; ++it) {
             const int abuf = it % nbufA;
-            int ok = 1;
-            if (lane == 0) {
-                if (ch == 0 && !wait(&a_full[abuf], (uint32_t)((it / nbufA) & 1))) ok = 0;
-                if (nchunks > 1 || j == 0) {
-                    if (!wait(&b_full[j % nbufB], (uint32_t)((j / nbufB) & 1))) ok = 0;
-                    else b_waited = j + 1;
-                }
-                if (j >= 2 && !wait(&d_empty[j & 1], (uint32_t)(((j - 2) >> 1) & 1))) ok = 0;
+            {
+                bool ok = wait(&a_full[abuf], (uint32_t)((it / nbufA) & 1));
+                if (it == 0 && !wait(&b_full, 0u)) ok = false;
+                if (it >= 2 && !wait(&d_empty[it & 1], (uint32_t)(((it - 2) >> 1) & 1))) ok = false;
+                ok = __all_sync(0xffffffffu, ok);
                 tc::fence_after_sync();
                 if (ok) {
-                    int k0, cnt;
-                    chunk_range(ch, k0, cnt);
-                    const uint32_t d_tmem = tbase + (uint32_t)((j & 1) * NW);
-                    const uint32_t idesc = tc::instr_desc(KIND, kTcTile, cnt * DP);
+                    const uint32_t d_tmem = tbase + (uint32_t)((it & 1) * NW);
+                    const uint32_t idesc = tc::instr_desc(KIND, kTcTile, chunk * DP);
                     const uint32_t a0 = tc::smem_u32(s_a + (size_t)abuf * NPART * A_PART);
-                    const uint32_t b0 = tc::smem_u32(s_b + (size_t)(j % nbufB) * CHUNK_BYTES);
+                    const uint32_t b0 = tc::smem_u32(s_b);
 #pragma unroll
                     for (int s = 0; s < KSTEPS; ++s) {
                         const uint64_t da = tc::smem_desc(a0 + s * 2 * LBO_A, LBO_A, 128);
                         const uint64_t db = tc::smem_desc(b0 + s * 2 * LBO_B, LBO_B, 128);
                         if (KIND == tc::kTF32) {
-                            tc::mma_tf32(d_tmem, da, db, idesc, s > 0);
+                            tc::mma_tf32_elect(d_tmem, da, db, idesc, s > 0);
                         } else {
-                            tc::mma(d_tmem, da, db, idesc, s > 0);
+                            tc::mma_elect(d_tmem, da, db, idesc, s > 0);
                             if (SPLIT == 3) {
                                 const uint64_t dal = tc::smem_desc(a0 + A_PART + s * 2 * LBO_A, LBO_A, 128);
                                 const uint64_t dbl = tc::smem_desc(b0 + chunk * B_COMP + s * 2 * LBO_B, LBO_B, 128);
-                                tc::mma(d_tmem, dal, db, idesc, true);
-                                tc::mma(d_tmem, da, dbl, idesc, true);
+                                tc::mma_elect(d_tmem, dal, db, idesc, true);
+                                tc::mma_elect(d_tmem, da, dbl, idesc, true);
                             }
                         }
                     }
                 }
                 // commits arrive when every earlier MMA has completed, issued or not
-                tc::commit(&d_full[j & 1]);
-                if (nchunks > 1) tc::commit(&b_empty[j % nbufB]);
-                if (ch == nchunks - 1) tc::commit(&a_empty[abuf]);
+                tc::commit_elect(&d_full[it & 1]);
+                tc::commit_elect(&a_empty[abuf]);
             }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            // operands of item j + nbufB - 1 go into the buffer MMA j - 1 has finished with
-            const int jn = j + nbufB - 1;
-            if (nchunks > 1 && j >= 1 && jn < J) {
-                int fine = 1;
-                if (lane == 0 && !wait(&b_empty[jn % nbufB], (uint32_t)(((jn - nbufB) / nbufB) & 1))) fine = 0;
-                fine = __shfl_sync(0xffffffffu, fine, 0);
-                if (fine) issue_b(jn);
-            }
+            __syncwarp();
         }
-        // drain: every requested copy has landed before the CTA exits
-        if (lane == 0)
-            for (int q = b_waited; q < b_issued; ++q) tc::mbar_wait(&b_full[q % nbufB], (uint32_t)((q / nbufB) & 1));
+        // the copy has landed before the CTA exits, whatever timed out
+        if (lane == 0 && my_tiles > 0) tc::mbar_wait(&b_full, 0u);
     } else if (warp < kFirstEpiWarp) {
         // ================= converters: sample tiles -> A operand =================
         const int ctid = tid - 32;
@@ -335,33 +251,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
         };
         for (int s = 0; s < S; ++s) issue_raw(s);
         const int row = ctid & (kTcTile - 1), half = ctid >> 7;
-        constexpr int HV = DP / 8;  // float4s of this thread's half row
         for (int it = 0; it < my_tiles; ++it) {
             const int64_t i = tile_of(it) * kTcTile + row;
             const bool active = i < p.n;
-            // DIRECT (no staged tile): this thread's half row straight from
-            // global memory into registers, issued before the A-buffer wait so
-            // its latency overlaps the previous tile's MMAs
-            float4 gv[DIRECT ? HV : 1];
-            if constexpr (DIRECT) {
-#pragma unroll
-                for (int u = 0; u < HV; ++u) {
-                    const int c = half * (DP / 2) + 4 * u;
-                    if (active && vec && c + 3 < p.d) {
-                        gv[u] = *reinterpret_cast<const float4 *>(p.x + i * p.d + c);
-                    } else {
-                        const float *xr = p.x + i * p.d;
-                        gv[u] = make_float4(active && c < p.d ? xr[c] : 0.f, active && c + 1 < p.d ? xr[c + 1] : 0.f,
-                                            active && c + 2 < p.d ? xr[c + 2] : 0.f,
-                                            active && c + 3 < p.d ? xr[c + 3] : 0.f);
-                    }
-                }
-            } else {
-                if (S == 1) tc::cp_async_wait<0>();
-                else if (S == 2) tc::cp_async_wait<1>();
-                else tc::cp_async_wait<2>();
-                tc::named_sync(1, kConvThreads);
-            }
+            tc::cp_async_wait<S - 1>();
+            tc::named_sync(1, kConvThreads);
             bool ok = true;
             const int abuf = it % nbufA;
             if (it >= nbufA) {
@@ -369,8 +263,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
                 ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
             }
             if (ok) {
-                const float *raw = S > 0 ? reinterpret_cast<const float *>(s_raw + (size_t)(it % S) * RAW_BYTES)
-                                         : nullptr;
+                const float *raw = reinterpret_cast<const float *>(s_raw + (size_t)(it % S) * RAW_BYTES);
                 unsigned char *a = s_a + (size_t)abuf * NPART * A_PART;
                 const bool full = active && p.d == DP;
 #pragma unroll
@@ -381,14 +274,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
                     for (int m = 0; m < PER; m += 4) {
                         const int c = q * PER + m;
                         const float4 cc = *reinterpret_cast<const float4 *>(s_c + c);
-                        if constexpr (DIRECT) {
-                            // gv holds zeros beyond d and for inactive rows
-                            const float4 f = gv[(qq * PER + m) / 4];
-                            v[m] = (active && c < p.d) ? f.x - cc.x : 0.f;
-                            v[m + 1] = (active && c + 1 < p.d) ? f.y - cc.y : 0.f;
-                            v[m + 2] = (active && c + 2 < p.d) ? f.z - cc.z : 0.f;
-                            v[m + 3] = (active && c + 3 < p.d) ? f.w - cc.w : 0.f;
-                        } else if (full) {
+                        if (full) {
                             const float4 f = *reinterpret_cast<const float4 *>(raw + row * RS + c);
                             v[m] = f.x - cc.x;
                             v[m + 1] = f.y - cc.y;
@@ -412,10 +298,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
             tc::fence_proxy_async();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&a_full[it % nbufA]);
-            if (!DIRECT) {
-                tc::named_sync(1, kConvThreads);  // the stage is consumed: refill it
-                issue_raw(it + S);
-            }
+            tc::named_sync(1, kConvThreads);  // the stage is consumed: refill it
+            issue_raw(it + S);
         }
         tc::cp_async_wait_all();
     } else {
@@ -423,19 +307,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
         const int qd = warp & 3;
         const int erow = 32 * qd + lane;
         const int ggen = (p.den_kind == ISSM_DENOM_PARTIAL) ? p.group[p.fixed_slot] : 0;
-        LseState<float> lse;
-        float gen_lq = 0.f, last_lq = 0.f, prev_ln = 0.f;
-        for (int j = 0; j < J; ++j) {
-            const int it = j / nchunks, ch = j - it * nchunks;
+        for (int it = 0; it < my_tiles; ++it) {
+            LseState<float> lse;
+            float gen_lq = 0.f, last_lq = 0.f, prev_ln = 0.f;
             const int64_t i = tile_of(it) * kTcTile + erow;
-            if (ch == 0 && p.mode == 1) prev_ln = i < p.n ? p.lognum[i] : 0.f;
-            const bool ok = __all_sync(0xffffffffu, wait(&d_full[j & 1], (uint32_t)((j >> 1) & 1)));
+            if (p.mode == 1) prev_ln = i < p.n ? p.lognum[i] : 0.f;
+            const bool ok = __all_sync(0xffffffffu, wait(&d_full[it & 1], (uint32_t)((it >> 1) & 1)));
             tc::fence_after_sync();
             if (ok) {
-                int k0, cnt;
-                chunk_range(ch, k0, cnt);
-                const uint32_t lane_base = tbase + ((uint32_t)(32 * qd) << 16) + (uint32_t)((j & 1) * NW);
-                for (int kk = 0; kk < cnt; ++kk) {
+                const uint32_t lane_base = tbase + ((uint32_t)(32 * qd) << 16) + (uint32_t)((it & 1) * NW);
+                for (int kk = 0; kk < chunk; ++kk) {
                     // a component's DP columns in one round trip (all loads, then one wait)
                     float v[DP];
                     if constexpr (DP == 64) tc::tmem_ld64(lane_base + (uint32_t)(kk * DP), v);
@@ -448,7 +329,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
                         r2b = fmaf(v[q + 1], v[q + 1], r2b);
                     }
                     const float r2 = r2a + r2b;
-                    const int k = k0 + kk;
+                    const int k = p.first_slot + kk;
                     float lq;
                     if (p.family == ISSM_GAUSSIAN) {
                         lq = p.lognorm[k] - 0.5f * r2;
@@ -466,8 +347,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
             }
             tc::fence_before_sync();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&d_empty[j & 1]);
-            if (ch != nchunks - 1) continue;
+            if (lane == 0) tc::mbar_arrive(&d_empty[it & 1]);
             if (ok && i < p.n) {
                 if (p.mode == 1) {
                     uint16_t reason = isnan(last_lq) ? ISSM_REASON_PROPOSAL_INVALID : 0;
@@ -488,16 +368,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
                     if (p.out_generating) p.out_generating[i] = bad ? -INFINITY : gen_lq;
                 }
             }
-            lse = LseState<float>();
-            gen_lq = 0.f;
-            last_lq = 0.f;
         }
     }
     // ---- every role is done; in-flight MMAs have completed before TMEM is freed ----
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (tid == 0 && abort_flag && J > 0) tc::mbar_wait(&d_full[(J - 1) & 1], (uint32_t)(((J - 1) >> 1) & 1));
+    if (tid == 0 && abort_flag && my_tiles > 0)
+        tc::mbar_wait(&d_full[(my_tiles - 1) & 1], (uint32_t)(((my_tiles - 1) >> 1) & 1));
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tbase, ncols);
 }
@@ -567,49 +445,23 @@ static int launch_tc(TcParams p, const float *w, const float *loc, int cslot, un
     const int nslots = p.last_slot - p.first_slot + 1;
     // one component centred at its own location: no offset column
     const bool nob = nslots == 1 && cslot == p.first_slot;
-    // largest chunk (<= 256 TMEM columns) whose buffers fit: one chunk keeps
-    // three staged tiles and two A buffers; several chunks keep one A buffer
-    // and a ring of kBRing chunk buffers, with one staged tile or none
-    int chunk = min(nslots, 256 / DP), nch = 1, stages = 1, bring = kBRing;
-    size_t smem = 0;
-    for (; chunk >= 1; --chunk) {
-        nch = (nslots + chunk - 1) / chunk;
-        if (nch == 1) {
-            stages = 3;
-            smem = stages * RAW_BYTES + (nob ? 3 * NPART * A_PART_NOB : 2 * NPART * A_PART) +
-                   (size_t)NPART * chunk * B_COMP + (size_t)DP * 4;
-        } else {
-            // a staged tile if it fits beside a kBRing-deep operand ring; else
-            // the converters read their rows from global memory (no staged
-            // tile), with a kBRing- or 2-deep ring, which leaves room for
-            // larger chunks (fewer, wider MMA items per tile)
-            const size_t base = NPART * A_PART + (size_t)DP * 4, cb = (size_t)NPART * chunk * B_COMP;
-            bring = kBRing;
-            stages = RAW_BYTES + base + kBRing * cb <= kTcMaxSmem ? 1 : 0;
-            if (stages == 0 && base + kBRing * cb > kTcMaxSmem) bring = 2;
-            smem = stages * RAW_BYTES + base + bring * cb;
-        }
-        if (smem <= kTcMaxSmem) break;
-    }
-    if (chunk < 1) return ISSM_E_UNSUPPORTED;
-    p.chunk = chunk;
-    p.nchunks = nch;
-    p.raw_stages = stages;
-    p.bring = bring;
-    { tc_prepare_kernel<KIND, SPLIT, DP><<<nslots, 256, 0, stream>>>(w, loc, p.d, p.first_slot, chunk, cslot, ops,
+    p.nslots = nslots;
+    // three staged tiles, two A buffers (three without the offset column) and
+    // every component's operands; more components than an accumulator's 256
+    // columns or the shared memory hold go to the paired tiles
+    const size_t smem = kRawStages * RAW_BYTES + (nob ? 3 * NPART * A_PART_NOB : 2 * NPART * A_PART) +
+                        (size_t)NPART * nslots * B_COMP + (size_t)DP * 4;
+    if (nslots * DP > 256 || smem > kTcMaxSmem) return launch_pair(KIND, DP, p, w, loc, cslot, ops, center, stream);
+    { tc_prepare_kernel<KIND, SPLIT, DP><<<nslots, 256, 0, stream>>>(w, loc, p.d, p.first_slot, nslots, cslot, ops,
                                                                        center);
       note_launch(); }
-    // DIRECT (no staged tile; converters read rows from global memory) is a
-    // separate instantiation so the staged form keeps its registers
-    auto kern = stages == 0 ? mixture_tc_kernel<KIND, SPLIT, DP, true, false>
-                : nob && nch == 1 ? mixture_tc_kernel<KIND, SPLIT, DP, false, true>
-                                  : mixture_tc_kernel<KIND, SPLIT, DP, false, false>;
+    auto kern = nob ? mixture_tc_kernel<KIND, SPLIT, DP, true> : mixture_tc_kernel<KIND, SPLIT, DP, false>;
     const int st = allow_dynamic_smem((const void *)kern);
     if (st) return st;
     int occ = 1;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTcThreads, smem);
     if (e != cudaSuccess) return (int)e;
-    const int nw2 = 2 * chunk * DP;
+    const int nw2 = 2 * nslots * DP;
     const int ncols = nw2 <= 32 ? 32 : nw2 <= 64 ? 64 : nw2 <= 128 ? 128 : nw2 <= 256 ? 256 : 512;
     occ = max(1, min(occ, 512 / ncols));  // TMEM allocations never wait
     p.ntiles = (int)((p.n + kTcTile - 1) / kTcTile);

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
     __shared__ float s_s0[kMtConvWarps];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tc::uniform_warp(), lane = tid & 31;
     if (warp == 0) tc::tmem_alloc(&tmem_base, 256);
     if (tid == 0) {
         for (int b = 0; b < kMtABufs; ++b) {
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tbase = tmem_base;  // D: 128 lanes x 144 columns
+    const uint32_t tbase = tc::uniform(tmem_base);  // D: 128 lanes x 144 columns
     const int64_t ntiles = (n + kMtTile - 1) / kMtTile;
     const int my_tiles = (int)((ntiles - (int64_t)blockIdx.x + gridDim.x - 1) / gridDim.x);
     auto tile_of = [&](int it) -> int64_t { return (int64_t)blockIdx.x + (int64_t)it * gridDim.x; };
@@ -146,18 +146,18 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
         constexpr uint32_t LBO = 128, SBO = kMtTile * 16;  // K-group stride, row-group stride
         for (int it = 0; it < my_tiles; ++it) {
             const int buf = it % kMtABufs;
-            if (lane == 0) {
-                const bool ok = wait(&a_full[buf], (uint32_t)((it / kMtABufs) & 1));
+            {
+                const bool ok = __all_sync(0xffffffffu, wait(&a_full[buf], (uint32_t)((it / kMtABufs) & 1)));
                 tc::fence_after_sync();
                 if (ok) {
                     const uint32_t a0 = tc::smem_u32(s_a + (size_t)buf * kMtBuf);
 #pragma unroll
                     for (int s = 0; s < kMtTile / 16; ++s) {
                         const uint64_t da = tc::smem_desc(a0 + s * 256, LBO, SBO);
-                        tc::mma(tbase, da, da, idesc, it > 0 || s > 0);
+                        tc::mma_elect(tbase, da, da, idesc, it > 0 || s > 0);
                     }
                 }
-                tc::commit(&a_empty[buf]);
+                tc::commit_elect(&a_empty[buf]);
             }
             __syncwarp();
         }

@@ -271,3 +271,37 @@ def test_resampling_kept_weights(issm, orc, cuda, n, dtype):
     assert np.array_equal(got, orc.resample_multinomial_fixed(lw.astype(np.float64), u))
     got = issm.ops.resample_systematic(tl, 0.37, 500).cpu().numpy()
     assert np.array_equal(got, orc.resample_systematic_fixed(lw.astype(np.float64), 0.37, 500))
+
+
+# The forms' bounds on a log density, as for the other tensor-core densities:
+# 5e-5 (BF16 x3) and 4e-3 (TF32) of max(1, |value|).
+@pytest.mark.parametrize("form,tol", [("bf16", 5e-5), ("tf32", 4e-3)])
+@pytest.mark.parametrize("n,d,k,dof", [(1, 64, 3, None), (127, 33, 5, None), (129, 64, 40, None), (255, 17, 9, 5.0),
+                                       (257, 32, 12, None), (513, 16, 17, None), (300, 1, 64, 4.0), (1000, 5, 33, None),
+                                       (40_001, 64, 7, None), (79_000, 15, 21, None), (200, 63, 4, 7.0)])
+def test_paired_tiles_density(issm, orc, cuda, form, tol, n, d, k, dof):
+    """More components than one accumulator holds: odd tile counts, partial
+    last chunks, several pairs per CTA, full, prefix and partial denominators."""
+    rng = np.random.default_rng(13 * d + k)
+    db, ob = _factor_bank(issm, orc, rng, d, k, np.float32, cuda, dof)
+    db.attach_inverse_factors()
+    x = (1.5 * rng.normal(size=(n, d))).astype(np.float32)
+    tx = torch.tensor(x, device=cuda)
+    prec = issm.native.PREC_BF16 if form == "bf16" else issm.native.PREC_TF32
+    coef = np.log(rng.dirichlet(np.ones(k))).astype(np.float32)
+    groups = (1 + np.arange(k) % 2).astype(np.int32)
+    tc, tg = torch.tensor(coef, device=cuda), torch.tensor(groups, device=cuda)
+    fixed = int(rng.integers(0, k))
+    for kind, okind in ((issm.native.DENOM_FULL, orc.DENOM_FULL), (issm.native.DENOM_PARTIAL, orc.DENOM_PARTIAL),
+                        (issm.native.DENOM_PREFIX, orc.DENOM_PREFIX)):
+        terms = k if kind == issm.native.DENOM_PREFIX else 0
+        den = issm.ops.denominator(kind, tc, terms=terms, groups=tg if kind == issm.native.DENOM_PARTIAL else None)
+        fail = issm.ops.new_failures(cuda)
+        got, gen = issm.ops.mixture_logdensity(db, den, tx, fixed_slot=fixed, failures=fail, generating=True,
+                                               precision=prec)
+        exp, egen, _ = orc.mixture_logdensity(ob, x.astype(np.float64).reshape(-1), okind, coef.astype(np.float64),
+                                              terms=terms, fixed_slot=fixed, group_of_slot=groups)
+        for a, b in ((got, exp), (gen, egen)):
+            assert np.all(np.abs(a.double().cpu().numpy() - b) <= tol * np.maximum(1.0, np.abs(b)))
+        assert int(fail[0].item()) == 0
+    issm.ops.check_tensor_core_errors(cuda)
