@@ -2,7 +2,6 @@
 // and the kernel translation units.
 #pragma once
 
-#include <cuda.h>  // CUtensorMap (types only; driver calls are resolved through the runtime)
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -69,10 +68,6 @@ int population_covariances(const void *x, int d, int dtype, const void *weights,
                            cudaStream_t stream);
 int population_factors(const void *covs, int d, int k, int dtype, const uint8_t *status, const void *dofs,
                        void *factors, int32_t *info, cudaStream_t stream);
-
-// tensor maps of n x d FP32 sample arrays, 32-float x 128-row boxes (tma.cu)
-bool row_tiles_supported(const void *x, int d, int64_t n);
-int encode_row_tiles(CUtensorMap *map, const void *x, int d, int64_t n);
 
 // one launch per phase across the in-flight runs of a serving loop (group.cu)
 int group_step(const void *runs, int nruns, int64_t blocks_new, int64_t blocks_all, int64_t blocks_mom,

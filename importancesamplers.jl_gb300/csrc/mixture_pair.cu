@@ -24,7 +24,7 @@
 // ran at 33 bytes of operands per clock and SM out of L2, 1,268 us for
 // 1,000,003 samples x 40 components, d = 64 (BF16x3); this form takes 769 us, and
 // 1,139 against 3,766 us for 4,194,304 x 64, d = 16. Tensor time is 1,418 clocks
-// per (pair, chunk) of d = 64, 300 us of the 769; the epilogue's TMEM reads and
+// per (pair, chunk) of d = 64, about 370 us of the 769; the epilogue's TMEM reads and
 // the handover between the two bound the rest. Few samples share the tiles out
 // worse (pairs, not tiles, per SM), yet 50,000 x 40, d = 64 still gains: 91 to
 // 79 us; x 8 is even at 35.5. Every wait is bounded; a

@@ -21,12 +21,16 @@
 //   tc_prepare_kernel  one CTA per slot: W_k in MMA operand form (bf16 hi/lo
 //                      or tf32, row-contiguous canonical layout) and b_k;
 //   mixture_tc_kernel  persistent, one 128-sample tile at a time:
-//     * warps 1-8 stream sample tiles with cp.async into a ring of padded
-//       stages and centre, round and split each into the A operand (two or
-//       three buffers, so converting tile t+1 overlaps MMAs of tile t);
+//     * warps 1-8 read the samples into registers and centre, round and split
+//       them into the A operand, groups of warps on alternate tiles;
 //     * warp 0 copies the operands once and issues the MMAs of a tile into one
 //       of two TMEM accumulators;
-//     * warps 9-12 (one per TMEM lane quadrant) run the epilogue of the other.
+//     * warps 9-16 reduce the accumulators, four (a TMEM lane quadrant each) per
+//       accumulator.
+// One component of 1,000,003 samples, d = 64: 70 us with the operand kernel (3.8
+// TB/s; reading alone is 40), 101 with rows staged by cp.async and one epilogue
+// warp per quadrant; four components 310 -> 115; d = 33, one component 173 -> 66;
+// d = 63 237 -> 81.
 // Every wait is bounded; a timeout sets the sticky error word and the CTA
 // unwinds after draining its outstanding copies and MMAs.
 #include "mixture_tc.cuh"
@@ -86,12 +90,16 @@ __global__ void __launch_bounds__(256) tc_prepare_kernel(const float *__restrict
 }
 
 // Warp roles of mixture_tc_kernel.
-constexpr int kConvWarps = 8;  // stage sample tiles and build the A operand
-constexpr int kEpiWarps = 4;   // one per TMEM lane quadrant
-constexpr int kConvThreads = 32 * kConvWarps;
+constexpr int kConvWarps = 8;  // read the samples and build the A operand
+constexpr int kEpiWarps = 8;   // per accumulator one per TMEM lane quadrant
 constexpr int kFirstEpiWarp = 1 + kConvWarps;
 constexpr int kTcThreads = 32 * (1 + kConvWarps + kEpiWarps);
-constexpr int kRawStages = 3;  // sample tiles staged ahead
+// Every converter warp holds 64 floats per lane, whatever DP: groups of warps on
+// alternate tiles, 64 KB of samples on their way per CTA. (All eight warps on one
+// tile with the next two prefetched was slower: the proxy fence after a tile's
+// stores waits for the loads issued before it.)
+__host__ __device__ constexpr int conv_groups(int DP) { return 128 / DP; }
+__host__ __device__ constexpr int tc_abufs(int DP) { return DP == 64 ? 3 : DP == 32 ? 6 : 10; }  // A operand buffers
 
 // NOB: one component centred at its own location, whose offset column
 // -W (mu - c) is therefore zero: the MMAs run over the coordinates' K groups
@@ -103,25 +111,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
     constexpr int KG = DP / PER;              // K groups of the sample coordinates
     constexpr int KGB = KG + 2;               // operand form: plus the offset column and padding
     constexpr int KGX = NOB ? KG : KGB;       // K groups the MMAs read
-    constexpr int QH = KG / 2;                // K groups converted per thread (two threads per row)
     constexpr int NPART = SPLIT == 3 ? 2 : 1;
-    constexpr int RS = DP + 4;                // padded raw row (floats): conflict-free row reads
-    constexpr int RAW_BYTES = kTcTile * RS * 4;
     constexpr int A_PART = kTcTile * KGX * 16;
     constexpr int B_COMP = DP * KGB * 16;
     constexpr int KSTEPS = KGX / 2;           // MMA K slices of 32 bytes
     constexpr uint32_t LBO_A = kTcTile * 16;
     const int chunk = p.nslots;  // components, all in one accumulator
-    constexpr int S = kRawStages, nbufA = NOB ? 3 : 2;
+    constexpr int nbufA = tc_abufs(DP), CG = conv_groups(DP);
     const uint32_t LBO_B = (uint32_t)(chunk * DP * 16);
     const uint32_t CHUNK_BYTES = (uint32_t)(NPART * chunk * B_COMP);
 
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *s_raw = smem;
-    unsigned char *s_a = s_raw + (size_t)S * RAW_BYTES;
+    unsigned char *s_a = smem;
     unsigned char *s_b = s_a + (size_t)nbufA * NPART * A_PART;
-    float *s_c = reinterpret_cast<float *>(s_b + CHUNK_BYTES);
-    __shared__ __align__(8) uint64_t a_full[3], a_empty[3], b_full, d_full[2], d_empty[2];
+    __shared__ __align__(8) uint64_t a_full[nbufA], a_empty[nbufA], b_full, d_full[2], d_empty[2];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
 
@@ -130,19 +133,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
     const uint32_t ncols = 2 * NW <= 32 ? 32 : 2 * NW <= 64 ? 64 : 2 * NW <= 128 ? 128 : 2 * NW <= 256 ? 256 : 512;
     if (warp == 0) tc::tmem_alloc(&tmem_base, ncols);
     if (tid == 0) {
-        for (int b = 0; b < 3; ++b) {
-            tc::mbar_init(&a_full[b], kConvWarps);
+        for (int b = 0; b < nbufA; ++b) {
+            tc::mbar_init(&a_full[b], kConvWarps / CG);
             tc::mbar_init(&a_empty[b], 1);
         }
         for (int b = 0; b < 2; ++b) {
             tc::mbar_init(&d_full[b], 1);
-            tc::mbar_init(&d_empty[b], kEpiWarps);
+            tc::mbar_init(&d_empty[b], kEpiWarps / 2);
         }
         tc::mbar_init(&b_full, 1);
         tc::fence_mbar_init();
         abort_flag = 0;
     }
-    for (int c = tid; c < DP; c += kTcThreads) s_c[c] = p.center[c];
     // constant K groups of the A buffers: a 1 in column DP (hi part), zeros elsewhere
     for (int e = tid; e < (NOB ? 0 : nbufA * NPART * 2 * kTcTile); e += kTcThreads) {
         const int row = e % kTcTile, g = (e / kTcTile) & 1, part = (e / (2 * kTcTile)) % NPART,
@@ -218,96 +220,66 @@ __global__ void __launch_bounds__(kTcThreads, 1) mixture_tc_kernel(TcParams p) {
         if (lane == 0 && my_tiles > 0) tc::mbar_wait(&b_full, 0u);
     } else if (warp < kFirstEpiWarp) {
         // ================= converters: sample tiles -> A operand =================
-        const int ctid = tid - 32;
-        const bool vec = (p.d % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.x) & 15) == 0);
-        auto issue_raw = [&](int it) {
-            if (it < my_tiles) {
-                const int64_t row0 = tile_of(it) * kTcTile;
-                const int rows = (int)min((int64_t)kTcTile, p.n - row0);
-                float *dst = reinterpret_cast<float *>(s_raw + (size_t)(it % S) * RAW_BYTES);
-                const float *src = p.x + row0 * p.d;
-                if (vec && p.d == DP) {
-                    constexpr int Q4 = DP / 4;
-                    const int total = rows * Q4;
-                    for (int e = ctid; e < total; e += kConvThreads) {
-                        const int r = e / Q4, c4 = e % Q4;
-                        tc::cp_async16(dst + r * RS + c4 * 4, src + (size_t)e * 4);
-                    }
-                } else if (vec) {
-                    const int q4 = p.d >> 2, total = rows * q4;
-                    for (int e = ctid; e < total; e += kConvThreads) {
-                        const int r = e / q4, c4 = e - r * q4;
-                        tc::cp_async16(dst + r * RS + c4 * 4, src + (size_t)r * p.d + c4 * 4);
-                    }
-                } else {
-                    const int total = rows * p.d;
-                    for (int e = ctid; e < total; e += kConvThreads) {
-                        const int r = e / p.d, c = e - r * p.d;
-                        tc::cp_async4(dst + r * RS + c, src + (size_t)r * p.d + c);
-                    }
-                }
+        // Groups of warps take alternate tiles. A warp converts RL rows x GL groups
+        // of 8 coordinates per pass, so a request's lanes read whole 32-byte sectors
+        // and eight lanes of a group store 128 contiguous operand bytes; the next
+        // tile of the group is requested as soon as this one's registers are free
+        constexpr int NG = DP / 8, GL = NG < 4 ? NG : 4, RL = 32 / GL, GP = NG / GL;
+        constexpr int WG = kConvWarps / CG, RW = kTcTile / WG, RP = RW / RL;  // warps of a group, rows of a warp
+        const int cw = (warp - 1) % WG, cgroup = (warp - 1) / WG, rl = lane % RL, gl = lane / RL;
+        const int access = row_access(p.x, p.d);
+        float cc[GP][8], v[RP][GP][8];
+#pragma unroll
+        for (int gp = 0; gp < GP; ++gp)
+#pragma unroll
+            for (int m = 0; m < 8; ++m) cc[gp][m] = p.center[(gp * GL + gl) * 8 + m];  // zero beyond d
+        auto load = [&](int it) {
+#pragma unroll
+            for (int rp = 0; rp < RP; ++rp) {
+                const int64_t i = tile_of(it) * kTcTile + RW * cw + rp * RL + rl;
+#pragma unroll
+                for (int gp = 0; gp < GP; ++gp)
+                    load_group(v[rp][gp], p.x, i, it < my_tiles && i < p.n, p.d, (gp * GL + gl) * 8, access);
             }
-            tc::cp_async_commit();
         };
-        for (int s = 0; s < S; ++s) issue_raw(s);
-        const int row = ctid & (kTcTile - 1), half = ctid >> 7;
-        for (int it = 0; it < my_tiles; ++it) {
-            const int64_t i = tile_of(it) * kTcTile + row;
-            const bool active = i < p.n;
-            tc::cp_async_wait<S - 1>();
-            tc::named_sync(1, kConvThreads);
-            bool ok = true;
+        load(cgroup);
+        for (int it = cgroup; it < my_tiles; it += CG) {
             const int abuf = it % nbufA;
-            if (it >= nbufA) {
-                if (lane == 0) ok = wait(&a_empty[abuf], (uint32_t)(((it - nbufA) / nbufA) & 1));
-                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-            }
+            const bool ok =
+                it < nbufA || __all_sync(0xffffffffu, wait(&a_empty[abuf], (uint32_t)(((it - nbufA) / nbufA) & 1)));
             if (ok) {
-                const float *raw = reinterpret_cast<const float *>(s_raw + (size_t)(it % S) * RAW_BYTES);
                 unsigned char *a = s_a + (size_t)abuf * NPART * A_PART;
-                const bool full = active && p.d == DP;
 #pragma unroll
-                for (int qq = 0; qq < QH; ++qq) {
-                    const int q = half * QH + qq;
-                    float v[PER];
+                for (int rp = 0; rp < RP; ++rp) {
+                    const int row = RW * cw + rp * RL + rl;
 #pragma unroll
-                    for (int m = 0; m < PER; m += 4) {
-                        const int c = q * PER + m;
-                        const float4 cc = *reinterpret_cast<const float4 *>(s_c + c);
-                        if (full) {
-                            const float4 f = *reinterpret_cast<const float4 *>(raw + row * RS + c);
-                            v[m] = f.x - cc.x;
-                            v[m + 1] = f.y - cc.y;
-                            v[m + 2] = f.z - cc.z;
-                            v[m + 3] = f.w - cc.w;
-                        } else {
-                            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (active) f = *reinterpret_cast<const float4 *>(raw + row * RS + c);
-                            v[m] = (active && c < p.d) ? f.x - cc.x : 0.f;
-                            v[m + 1] = (active && c + 1 < p.d) ? f.y - cc.y : 0.f;
-                            v[m + 2] = (active && c + 2 < p.d) ? f.z - cc.z : 0.f;
-                            v[m + 3] = (active && c + 3 < p.d) ? f.w - cc.w : 0.f;
+                    for (int gp = 0; gp < GP; ++gp) {
+                        float z[8];
+#pragma unroll
+                        for (int m = 0; m < 8; ++m) z[m] = v[rp][gp][m] - cc[gp][m];
+#pragma unroll
+                        for (int h = 0; h < 8 / PER; ++h) {
+                            const int q = (gp * GL + gl) * (8 / PER) + h;
+                            const uint4 hi = pack_hi<KIND>(z + h * PER);
+                            *reinterpret_cast<uint4 *>(a + (size_t)q * LBO_A + row * 16) = hi;
+                            if (NPART == 2)
+                                *reinterpret_cast<uint4 *>(a + A_PART + (size_t)q * LBO_A + row * 16) =
+                                    pack_lo(z + h * PER, hi);
                         }
                     }
-                    const uint4 hi = pack_hi<KIND>(v);
-                    *reinterpret_cast<uint4 *>(a + (size_t)q * LBO_A + row * 16) = hi;
-                    if (NPART == 2)
-                        *reinterpret_cast<uint4 *>(a + A_PART + (size_t)q * LBO_A + row * 16) = pack_lo(v, hi);
                 }
             }
             tc::fence_proxy_async();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&a_full[it % nbufA]);
-            tc::named_sync(1, kConvThreads);  // the stage is consumed: refill it
-            issue_raw(it + S);
+            if (lane == 0) tc::mbar_arrive(&a_full[abuf]);
+            load(it + CG);
         }
-        tc::cp_async_wait_all();
     } else {
         // ================= epilogue: radial densities and the log-sum-exp =================
-        const int qd = warp & 3;
+        const int qd = warp & 3, group = (warp - kFirstEpiWarp) >> 2;
         const int erow = 32 * qd + lane;
         const int ggen = (p.den_kind == ISSM_DENOM_PARTIAL) ? p.group[p.fixed_slot] : 0;
-        for (int it = 0; it < my_tiles; ++it) {
+        for (int it = group; it < my_tiles; it += 2) {  // accumulator `group`
             LseState<float> lse;
             float gen_lq = 0.f, last_lq = 0.f, prev_ln = 0.f;
             const int64_t i = tile_of(it) * kTcTile + erow;
@@ -437,7 +409,6 @@ static int launch_tc(TcParams p, const float *w, const float *loc, int cslot, un
     constexpr int EB = KIND == tc::kBF16 ? 2 : 4;
     constexpr int KGX = DP * EB / 16 + 2;
     constexpr int NPART = SPLIT == 3 ? 2 : 1;
-    constexpr size_t RAW_BYTES = (size_t)kTcTile * (DP + 4) * 4;
     constexpr size_t A_PART = (size_t)kTcTile * KGX * 16;
     constexpr size_t A_PART_NOB = (size_t)kTcTile * (KGX - 2) * 16;
     constexpr size_t B_COMP = (size_t)DP * KGX * 16;
@@ -446,12 +417,12 @@ static int launch_tc(TcParams p, const float *w, const float *loc, int cslot, un
     // one component centred at its own location: no offset column
     const bool nob = nslots == 1 && cslot == p.first_slot;
     p.nslots = nslots;
-    // three staged tiles, two A buffers (three without the offset column) and
-    // every component's operands; more components than an accumulator's 256
-    // columns or the shared memory hold go to the paired tiles
-    const size_t smem = kRawStages * RAW_BYTES + (nob ? 3 * NPART * A_PART_NOB : 2 * NPART * A_PART) +
-                        (size_t)NPART * nslots * B_COMP + (size_t)DP * 4;
-    if (nslots * DP > 256 || smem > kTcMaxSmem) return launch_pair(KIND, DP, p, w, loc, cslot, ops, center, stream);
+    // the A buffers and every component's operands; more components than an
+    // accumulator's 256 columns hold go to the paired tiles
+    const size_t smem = (size_t)tc_abufs(DP) * NPART * (nob ? A_PART_NOB : A_PART) + (size_t)NPART * nslots * B_COMP;
+    static_assert((size_t)tc_abufs(DP) * NPART * A_PART + (size_t)NPART * (256 / DP) * B_COMP <= kTcMaxSmem,
+                  "shared memory per CTA");
+    if (nslots * DP > 256) return launch_pair(KIND, DP, p, w, loc, cslot, ops, center, stream);
     { tc_prepare_kernel<KIND, SPLIT, DP><<<nslots, 256, 0, stream>>>(w, loc, p.d, p.first_slot, nslots, cslot, ops,
                                                                        center);
       note_launch(); }

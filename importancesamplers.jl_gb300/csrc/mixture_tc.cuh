@@ -5,6 +5,7 @@
 
 #include "issm_device.cuh"
 #include "issm_internal.h"
+#include "sample_rows.cuh"
 #include "tcgen05.cuh"
 
 namespace issm {

@@ -22,60 +22,44 @@
 // kernels are always launched (graph replays see a fixed sequence) and
 // return at once when the flag is clear.
 //
-// A is stored MN-major: each sample's 8-coordinate groups are 16-byte chunks,
-// so four threads convert a sample row straight from the staged tile. Warp
-// roles: warp 0 issues the MMAs; warps 1..16 build the operand (three
-// buffers, so conversion runs up to two tiles ahead of the MMAs) from the
-// staged tiles; warp 17 stages the tiles. For d = 32 or 64 (aligned arrays)
-// the stager keeps a three-deep ring of stages filled by tensor copies
-// (cp.async.bulk.tensor through a tensor map of the samples: one or two
-// 32-float x 128-row boxes per tile, 128-byte swizzle, so converters read
-// rows without bank conflicts, plus one bulk copy of the tile's log weights;
-// completion counted in bytes on the stage's mbarrier); converters wait on
-// that mbarrier and release the stage with one arrival per warp, so no role
-// ever waits on a CTA-wide barrier. Other shapes stage padded rows with
-// cp.async from the converters. Per-CTA partials are summed across CTAs
-// (compensated FP32) and mean = c + S1/S0, cov = S2/S0 - (S1/S0)(S1/S0)^T in
-// FP64.
-#include <cstring>
-
+// A is stored MN-major: each sample's 8-coordinate groups are 16-byte chunks, so
+// a lane converts a group straight from its registers. Warp roles: warp 0 issues
+// the MMAs; warps 1..12 read, weight and split the samples, three groups of four
+// warps on alternate tiles, each lane's next 64 floats requested as soon as the
+// last ones are converted (96 KB on their way per CTA). Per-CTA partials are summed
+// across CTAs (compensated FP32) and mean = c + S1/S0, cov = S2/S0 - (S1/S0)
+// (S1/S0)^T in FP64.
+//
+// The pass is bound by reading the samples: 64 us on average over 50,000 ..
+// 2,000,000 samples of d = 64, 4.3 TB/s with the launch. Sixteen converter warps
+// in lockstep on tiles staged by tensor copies took 66; for d other than 32 and
+// 64, where they staged padded rows by cp.async, up to 2.5 times as long (d = 33,
+// 100,000 .. 1,000,000 samples: 77 us, now 29). Sixteen warps of this form took
+// 71: 17 warps leave 96 registers a thread, and they spill.
 #include "issm_device.cuh"
 #include "issm_internal.h"
+#include "sample_rows.cuh"
 #include "tcgen05.cuh"
 
 namespace issm {
 
-// 16 converter warps (four threads per sample row, two coordinate groups
-// each): the conversion is latency-bound, and with one CTA per SM (shared
-// memory) only more warps hide its dependency chains
-constexpr int kMtConvWarps = 16;
-constexpr int kMtConvThreads = 32 * kMtConvWarps;
-constexpr int kMtStagerWarp = 1 + kMtConvWarps;
-constexpr int kMtThreads = 32 * (2 + kMtConvWarps);  // issuer, converters, stager
+constexpr int kMtConvWarps = 12;
+constexpr int kMtThreads = 32 * (1 + kMtConvWarps);  // issuer, converters
+constexpr int kMtConvGroups = 3;  // groups of four warps, each on its own tile
 constexpr int kMtTile = 128;   // samples per tile = MMA K extent per tile
-constexpr int kMtTPR = kMtConvThreads / kMtTile;  // converter threads per sample row
-constexpr int kMtGPT = 8 / kMtTPR;                // coordinate groups (of 8) per converter thread
-constexpr int kMtCtasPerSm = 1;  // CTAs per SM (two 64-sample pipelines measured the same)
+constexpr int kMtCtasPerSm = 1;
 constexpr int kMtCols = 80;    // columns of a CTA's partial (64 coordinates, sqrt(w), padding)
 constexpr int kMtN = 144;      // MMA N: hi rows, lo rows, sqrt(w) hi and lo, padding
-constexpr int kMtStages = 3;   // staged sample tiles in flight
-constexpr int kMtABufs = 3;    // operand buffers: conversion runs up to two tiles ahead of the MMAs
-constexpr int kMtRS = 68;      // padded row of a staged tile (floats): conflict-free row reads
-constexpr int kMtWOff = kMtTile * kMtRS * 4;  // byte offset of the tile's log weights in a stage
-// rows (padded, or two swizzled boxes), then the log weights; a 1024-byte multiple
-constexpr int kMtRawBytes = (kMtWOff + kMtTile * 4 + 1023) / 1024 * 1024;
+constexpr int kMtABufs = 6;    // operand buffers
 // One operand buffer holds 18 row groups of 128 samples x 16 bytes, MN-major:
 // groups 0..7 the bf16 hi parts of the 64 coordinates, groups 8..15 their lo
 // parts, group 16 (sqrt(w) hi, sqrt(w) lo, zeros) and group 17 zeros. A is
 // its first 16 groups (M = 128), B all 18 (N = 144).
 constexpr int kMtGroups = 18;
 constexpr int kMtBuf = kMtGroups * kMtTile * 16;
-// operand buffers, stages (1024-byte multiples: the swizzled boxes need 1024-byte
-// aligned destinations), centre; plus 1024 bytes to align the base
-constexpr size_t kMtSmem = (size_t)kMtABufs * kMtBuf + (size_t)kMtStages * kMtRawBytes + 256 + 1024;
+constexpr size_t kMtSmem = (size_t)kMtABufs * kMtBuf;
 static_assert(kMtSmem <= 232448 - 2048, "dynamic shared memory per CTA");
-static_assert(kMtBuf % 1024 == 0 && kMtRawBytes % 1024 == 0, "stages start on 1024-byte boundaries");
-static_assert(128 * 65 * 4 <= kMtRawBytes, "the epilogue's row sums fit in one stage");
+static_assert(128 * 65 * 4 <= kMtBuf, "the epilogue's row sums fit in one operand buffer");
 constexpr int kMtPartial = 65 * kMtCols;  // P = S / 2 of one CTA (the reduce forms S = P + P^T)
 
 __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(const float *__restrict__ x, int d, int64_t n,
@@ -83,17 +67,10 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
                                                                     const double *__restrict__ summary,
                                                                     const double *__restrict__ center,
                                                                     float *__restrict__ partial, int *error,
-                                                                    const int *__restrict__ gate,
-                                                                    const __grid_constant__ CUtensorMap tmap,
-                                                                    int tma) {
+                                                                    const int *__restrict__ gate) {
     if (gate != nullptr && *gate == 0) return;  // refinement pass not needed
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    // the swizzled boxes need 1024-byte aligned stages
-    unsigned char *smem = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
-    unsigned char *s_a = smem;                                    // [buf] x kMtBuf
-    unsigned char *s_raw = smem + (size_t)kMtABufs * kMtBuf;
-    float *s_c = reinterpret_cast<float *>(s_raw + (size_t)kMtStages * kMtRawBytes);
-    __shared__ __align__(8) uint64_t a_full[kMtABufs], a_empty[kMtABufs], raw_full[kMtStages], raw_empty[kMtStages];
+    extern __shared__ __align__(1024) unsigned char s_a[];  // [buf] x kMtBuf
+    __shared__ __align__(8) uint64_t a_full[kMtABufs], a_empty[kMtABufs];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
     __shared__ float s_s0[kMtConvWarps];
@@ -101,17 +78,12 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
     if (warp == 0) tc::tmem_alloc(&tmem_base, 256);
     if (tid == 0) {
         for (int b = 0; b < kMtABufs; ++b) {
-            tc::mbar_init(&a_full[b], kMtConvWarps);
+            tc::mbar_init(&a_full[b], kMtConvWarps / kMtConvGroups);
             tc::mbar_init(&a_empty[b], 1);
-        }
-        for (int s = 0; s < kMtStages; ++s) {
-            tc::mbar_init(&raw_full[s], 1);
-            tc::mbar_init(&raw_empty[s], kMtConvWarps);
         }
         tc::fence_mbar_init();
         abort_flag = 0;
     }
-    for (int c = tid; c < 64; c += kMtThreads) s_c[c] = c < d ? (float)center[c] : 0.f;
     // group 17 of every buffer: zeros (B rows 136..143, never read back)
     for (int e = tid; e < kMtABufs * kMtTile; e += kMtThreads)
         *reinterpret_cast<uint4 *>(s_a + (size_t)(e / kMtTile) * kMtBuf + 17 * kMtTile * 16 + (e % kMtTile) * 16) =
@@ -127,7 +99,6 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
     const int64_t ntiles = (n + kMtTile - 1) / kMtTile;
     const int my_tiles = (int)((ntiles - (int64_t)blockIdx.x + gridDim.x - 1) / gridDim.x);
     auto tile_of = [&](int it) -> int64_t { return (int64_t)blockIdx.x + (int64_t)it * gridDim.x; };
-    auto tile_rows = [&](int it) -> int { return (int)min((int64_t)kMtTile, n - tile_of(it) * kMtTile); };
     auto wait = [&](uint64_t *bar, uint32_t parity) -> bool {
         if (abort_flag) return false;
         if (tc::mbar_wait(bar, parity)) return true;
@@ -135,11 +106,6 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
         abort_flag = 1;
         return false;
     };
-    // tensor copies of the tiles (d = 32 or 64, aligned arrays; the host
-    // encoded the tensor map); else padded rows by cp.async
-    const bool bulk = tma != 0;
-    const int nbox = d > 32 ? 2 : 1;
-
     if (warp == 0) {
         // ---- issuer: D += [Ah; Al] [Ah; Al; sqrt(w)]^T, one MMA per K slice ----
         const uint32_t idesc = tc::instr_desc(tc::kBF16, 128, kMtN) | tc::kMajorMN;
@@ -161,164 +127,73 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
             }
             __syncwarp();
         }
-    } else if (warp == kMtStagerWarp) {
-        // ---- stager: the tile's one or two swizzled boxes by tensor copies,
-        // its log weights (whole 16-byte groups) by one bulk copy ----
-        if (bulk) {
-            int issued = 0;
-            for (int it = 0; it < my_tiles; ++it) {
-                const int s = it % kMtStages;
-                if (it >= kMtStages) {
-                    int ok = 1;
-                    if (lane == 0) ok = wait(&raw_empty[s], (uint32_t)(((it / kMtStages) - 1) & 1));
-                    if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-                }
-                const int64_t row0 = tile_of(it) * kMtTile;
-                const int rows = tile_rows(it);
-                const uint32_t wb = (uint32_t)(rows & ~3) * 4u;
-                unsigned char *dst = s_raw + (size_t)s * kMtRawBytes;
-                if (lane == 0) {
-                    // a box counts all its bytes (rows past n arrive as zeros)
-                    tc::mbar_arrive_expect_tx(&raw_full[s], (uint32_t)nbox * 16384u + wb);
-                    for (int b = 0; b < nbox; ++b)
-                        tc::tma_load_2d(dst + (size_t)b * 16384, &tmap, 32 * b, (int)row0, &raw_full[s]);
-                    if (wb > 0) tc::bulk_copy_g2s(dst + kMtWOff, lw + row0, wb, &raw_full[s]);
-                }
-                __syncwarp();
-                issued = it + 1;
-            }
-            // every copy lands before the CTA can exit (the converters consume
-            // them all unless a wait timed out)
-            if (lane == 0)
-                for (int it = max(0, issued - kMtStages); it < issued; ++it)
-                    tc::mbar_wait(&raw_full[it % kMtStages], (uint32_t)((it / kMtStages) & 1));
-        }
     } else {
-        // ---- converters: build [Ah; Al; sqrt(w)] from the staged tiles ----
-        const int ctid = tid - 32;
-        auto issue_raw = [&](int it) {  // cp.async staging (shapes without tensor copies)
-            if (it < my_tiles) {
-                const int64_t row0 = tile_of(it) * kMtTile;
-                const int rows = tile_rows(it);
-                float *dst = reinterpret_cast<float *>(s_raw + (size_t)(it % kMtStages) * kMtRawBytes);
-                float *dlw = dst + kMtTile * kMtRS;
-                const float *src = x + row0 * d;
-                const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-                if (vec) {
-                    const int q4 = d >> 2, total = rows * q4;
-                    for (int e = ctid; e < total; e += kMtConvThreads) {
-                        const int r = e / q4, c4 = e - r * q4;
-                        tc::cp_async16(dst + r * kMtRS + c4 * 4, src + (size_t)r * d + c4 * 4);
-                    }
-                } else {
-                    for (int e = ctid; e < rows * d; e += kMtConvThreads) {
-                        const int r = e / d, c = e - r * d;
-                        tc::cp_async4(dst + r * kMtRS + c, src + (size_t)r * d + c);
-                    }
-                }
-                for (int r = ctid; r < rows; r += kMtConvThreads) tc::cp_async4(dlw + r, lw + row0 + r);
-            }
-            tc::cp_async_commit();
-        };
-        if (!bulk)
-            for (int s = 0; s < kMtStages; ++s) issue_raw(s);
-        const int k = ctid % kMtTile, part = ctid / kMtTile;
-        float s0 = 0.f;  // sum of (sqrt(w) hi + lo)^2 over this thread's samples: S0 of the split operand
-        for (int it = 0; it < my_tiles; ++it) {
-            const int buf = it % kMtABufs, stage = it % kMtStages;
-            bool ok = true;
-            if (bulk) {
-                // every lane acquires the stage's bytes itself; the outcome is made warp-uniform
-                ok = __all_sync(0xffffffffu, wait(&raw_full[stage], (uint32_t)((it / kMtStages) & 1)));
-            } else {
-                tc::cp_async_wait<kMtStages - 1>();
-                tc::named_sync(1, kMtConvThreads);
-            }
-            if (it >= kMtABufs && ok) {
-                if (lane == 0) ok = wait(&a_empty[buf], (uint32_t)(((it / kMtABufs) - 1) & 1));
-                ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-            }
-            if (ok) {
-                const unsigned char *stage_p = s_raw + (size_t)stage * kMtRawBytes;
-                const float *raw = reinterpret_cast<const float *>(stage_p);
-                // coordinates c .. c + 3 of this thread's row: swizzled box or padded row
-                auto row_at = [&](int c) -> const float4 * {
-                    return reinterpret_cast<const float4 *>(bulk ? tc::swizzled_row_chunk(stage_p, k, c)
-                                                                 : raw + k * kMtRS + c);
-                };
-                unsigned char *ab = s_a + (size_t)buf * kMtBuf;
-                const int64_t i = tile_of(it) * kMtTile + k;
-                const bool active = i < n;
-                // the bulk copy carries whole 16-byte groups of weights; the
-                // (at most three) beyond them come from global memory
-                const int staged_w = bulk ? (tile_rows(it) & ~3) : kMtTile;
-                const float l = !active ? -INFINITY : (k < staged_w ? raw[kMtWOff / 4 + k] : lw[i]);
-                const float sw = l == -INFINITY ? 0.f : expf(0.5f * (l - m)) * inv_sqrt_s;
-                const bool full = active && d == 64;
+        // ---- converters: groups of four warps take alternate tiles; a warp's 32
+        // rows in four passes of 8, lane = row + 8 x group of 8 coordinates ----
+        constexpr int RP = 4;
+        const int cw = (warp - 1) & 3, cgroup = (warp - 1) >> 2, rl = lane & 7, gl = lane >> 3;
+        const int access = row_access(x, d);
+        float cc[2][8], v[RP][2][8], l[RP];
 #pragma unroll
-                for (int gg = 0; gg < kMtGPT; ++gg) {
-                    const int g = part * kMtGPT + gg, c = g * 8;
-                    float v[8];
-                    const float4 c0 = *reinterpret_cast<const float4 *>(s_c + c),
-                                 c1 = *reinterpret_cast<const float4 *>(s_c + c + 4);
-                    if (full) {
-                        const float4 f0 = *row_at(c);
-                        const float4 f1 = *row_at(c + 4);
-                        v[0] = sw * (f0.x - c0.x);
-                        v[1] = sw * (f0.y - c0.y);
-                        v[2] = sw * (f0.z - c0.z);
-                        v[3] = sw * (f0.w - c0.w);
-                        v[4] = sw * (f1.x - c1.x);
-                        v[5] = sw * (f1.y - c1.y);
-                        v[6] = sw * (f1.z - c1.z);
-                        v[7] = sw * (f1.w - c1.w);
-                    } else {
-                        float4 f0 = make_float4(0.f, 0.f, 0.f, 0.f), f1 = f0;
-                        if (active) {
-                            f0 = *row_at(c);
-                            f1 = *row_at(c + 4);
-                        }
-                        v[0] = (active && c < d) ? sw * (f0.x - c0.x) : 0.f;
-                        v[1] = (active && c + 1 < d) ? sw * (f0.y - c0.y) : 0.f;
-                        v[2] = (active && c + 2 < d) ? sw * (f0.z - c0.z) : 0.f;
-                        v[3] = (active && c + 3 < d) ? sw * (f0.w - c0.w) : 0.f;
-                        v[4] = (active && c + 4 < d) ? sw * (f1.x - c1.x) : 0.f;
-                        v[5] = (active && c + 5 < d) ? sw * (f1.y - c1.y) : 0.f;
-                        v[6] = (active && c + 6 < d) ? sw * (f1.z - c1.z) : 0.f;
-                        v[7] = (active && c + 7 < d) ? sw * (f1.w - c1.w) : 0.f;
+        for (int gg = 0; gg < 2; ++gg)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int c = (gl + 4 * gg) * 8 + j;
+                cc[gg][j] = c < d ? (float)center[c] : 0.f;
+            }
+        auto load = [&](int it) {
+#pragma unroll
+            for (int rp = 0; rp < RP; ++rp) {
+                const int64_t i = tile_of(it) * kMtTile + 32 * cw + 8 * rp + rl;
+                const bool active = it < my_tiles && i < n;
+                l[rp] = active ? lw[i] : -INFINITY;
+#pragma unroll
+                for (int gg = 0; gg < 2; ++gg) load_group(v[rp][gg], x, i, active, d, (gl + 4 * gg) * 8, access);
+            }
+        };
+        load(cgroup);
+        float s0 = 0.f;  // sum of (sqrt(w) hi + lo)^2 over this thread's samples: S0 of the split operand
+        for (int it = cgroup; it < my_tiles; it += kMtConvGroups) {
+            const int buf = it % kMtABufs;
+            const bool ok = it < kMtABufs ||
+                            __all_sync(0xffffffffu, wait(&a_empty[buf], (uint32_t)(((it / kMtABufs) - 1) & 1)));
+            if (ok) {
+#pragma unroll
+                for (int rp = 0; rp < RP; ++rp) {
+                    unsigned char *ab = s_a + (size_t)buf * kMtBuf + (32 * cw + 8 * rp + rl) * 16;
+                    const float sw = l[rp] == -INFINITY ? 0.f : expf(0.5f * (l[rp] - m)) * inv_sqrt_s;
+#pragma unroll
+                    for (int gg = 0; gg < 2; ++gg) {
+                        float z[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) z[j] = sw * (v[rp][gg][j] - cc[gg][j]);
+                        const uint4 hi = make_uint4(tc::pack_bf16x2(z[0], z[1]), tc::pack_bf16x2(z[2], z[3]),
+                                                    tc::pack_bf16x2(z[4], z[5]), tc::pack_bf16x2(z[6], z[7]));
+                        auto lo2 = [](float p, float q, uint32_t h) {
+                            return tc::pack_bf16x2(p - __uint_as_float(h << 16), q - __uint_as_float(h & 0xffff0000u));
+                        };
+                        const uint4 lo = make_uint4(lo2(z[0], z[1], hi.x), lo2(z[2], z[3], hi.y),
+                                                    lo2(z[4], z[5], hi.z), lo2(z[6], z[7], hi.w));
+                        *reinterpret_cast<uint4 *>(ab + (size_t)(gl + 4 * gg) * kMtTile * 16) = hi;
+                        *reinterpret_cast<uint4 *>(ab + (size_t)(8 + gl + 4 * gg) * kMtTile * 16) = lo;
                     }
-                    const uint4 hi = make_uint4(tc::pack_bf16x2(v[0], v[1]), tc::pack_bf16x2(v[2], v[3]),
-                                                tc::pack_bf16x2(v[4], v[5]), tc::pack_bf16x2(v[6], v[7]));
-                    auto lo2 = [](float a, float b, uint32_t h) {
-                        return tc::pack_bf16x2(a - __uint_as_float(h << 16), b - __uint_as_float(h & 0xffff0000u));
-                    };
-                    const uint4 lo = make_uint4(lo2(v[0], v[1], hi.x), lo2(v[2], v[3], hi.y), lo2(v[4], v[5], hi.z),
-                                                lo2(v[6], v[7], hi.w));
-                    *reinterpret_cast<uint4 *>(ab + (size_t)g * kMtTile * 16 + k * 16) = hi;
-                    *reinterpret_cast<uint4 *>(ab + (size_t)(8 + g) * kMtTile * 16 + k * 16) = lo;
-                }
-                if (part == kMtTPR - 1) {
-                    // group 16: sqrt(w) hi in row 128, its lo part in row 129
-                    const uint32_t h = tc::pack_bf16x2(sw, 0.f);
-                    const float swh = __uint_as_float(h << 16);
-                    const uint32_t hl = tc::pack_bf16x2(swh, sw - swh);
-                    const float swl = __uint_as_float(hl & 0xffff0000u);
-                    const float sws = swh + swl;  // exact: swl is a bf16 below swh's last bit
-                    s0 = fmaf(sws, sws, s0);
-                    *reinterpret_cast<uint4 *>(ab + (size_t)16 * kMtTile * 16 + k * 16) = make_uint4(hl, 0u, 0u, 0u);
+                    if (gl == 0) {
+                        // group 16: sqrt(w) hi in row 128, its lo part in row 129
+                        const uint32_t h = tc::pack_bf16x2(sw, 0.f);
+                        const float swh = __uint_as_float(h << 16);
+                        const uint32_t hl = tc::pack_bf16x2(swh, sw - swh);
+                        const float swl = __uint_as_float(hl & 0xffff0000u);
+                        const float sws = swh + swl;  // exact: swl is a bf16 below swh's last bit
+                        s0 = fmaf(sws, sws, s0);
+                        *reinterpret_cast<uint4 *>(ab + (size_t)16 * kMtTile * 16) = make_uint4(hl, 0u, 0u, 0u);
+                    }
                 }
             }
             tc::fence_proxy_async();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&a_full[buf]);
-            if (bulk) {
-                if (lane == 0) tc::mbar_arrive(&raw_empty[stage]);  // this warp is done with the stage
-            } else {
-                tc::named_sync(1, kMtConvThreads);  // the stage is consumed: refill it
-                issue_raw(it + kMtStages);
-            }
+            load(it + kMtConvGroups);
         }
-        if (!bulk) tc::cp_async_wait_all();
         // S0 per warp in a fixed order (lanes by xor tree, warps summed in order below)
         for (int off = 16; off > 0; off >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, off);
         if (lane == 0) s_s0[warp - 1] = s0;
@@ -337,8 +212,8 @@ __global__ void __launch_bounds__(kMtThreads, kMtCtasPerSm) moments_tc_kernel(co
     tc::fence_after_sync();
     float *out = partial + (size_t)blockIdx.x * kMtPartial;
     // row sums T[r][j] = D[r][j] + D[r][64 + j] (j < 64) and T[r][64] =
-    // D[r][128] + D[r][129] in the first stage's space (every copy has landed)
-    float *T = reinterpret_cast<float *>(s_raw);
+    // D[r][128] + D[r][129] in the first operand buffer's space (every MMA is done)
+    float *T = reinterpret_cast<float *>(s_a);
     // warps 1..4 read TMEM lane quadrants 1, 2, 3, 0 (a warp reads quadrant warp % 4)
     if (!abort_flag && warp >= 1 && warp <= 4) {
         const int q = warp & 3, row = 32 * q + lane;
@@ -506,23 +381,15 @@ int moments_tc(const void *x, int d, int64_t n, const void *lw, const double *su
     unsigned *counter = reinterpret_cast<unsigned *>(error + 1);  // zero with the workspace; reset by each use
     const int rblocks = (kMtPartial + 31) / 32;
     // pass 1 about `shift`
-    // tensor copies of the tiles when the shape allows (one map per call; both passes read it)
-    CUtensorMap tmap;
-    memset(&tmap, 0, sizeof(tmap));
-    int tma = 0;
-    if (row_tiles_supported(x, d, n) && ((reinterpret_cast<uintptr_t>(lw) & 15) == 0))
-        tma = encode_row_tiles(&tmap, x, d, n) == ISSM_OK ? 1 : 0;
     { moments_tc_kernel<<<blocks, kMtThreads, kMtSmem, stream>>>((const float *)x, d, n, (const float *)lw,
-                                                                       summary, shift, partial, error, nullptr,
-                                                                       tmap, tma);
+                                                                       summary, shift, partial, error, nullptr);
       note_launch(); }
     { moments_tc_reduce_kernel<<<rblocks, kMtReduceThreads, 0, stream>>>(partial, blocks, sums, d, shift, mean, cov,
                                                                          nullptr, refine, prev_factor, counter);
       note_launch(); }
     // pass 2 about the new mean (kernels return at once unless pass 1 set `refine`)
     { moments_tc_kernel<<<blocks, kMtThreads, kMtSmem, stream>>>((const float *)x, d, n, (const float *)lw,
-                                                                      summary, mean, partial, error, refine, tmap,
-                                                                      tma);
+                                                                      summary, mean, partial, error, refine);
       note_launch(); }
     { moments_tc_reduce_kernel<<<rblocks, kMtReduceThreads, 0, stream>>>(partial, blocks, sums, d, mean, mean, cov,
                                                                          refine, nullptr, nullptr, counter);
