@@ -379,12 +379,21 @@ __global__ void __launch_bounds__(256) fit_factor_kernel(const double *__restric
     __syncthreads();
     constexpr int LDI = 65;
     float *Lf = reinterpret_cast<float *>(A + dd);  // FP32 copy of the stored factor for the inverse
-    for (int e = tid; e < dd; e += 256) {
-        const int r = e % d, c = e / d;
-        const T v = r > c ? (T)(A[e] * s_scale[c]) : r == c ? (T)s_scale[c] : T(0);
-        out_factor[e] = v;
-        if (out_inverse != nullptr) Lf[r * LDI + c] = (float)v;
-        if (r > c) invalid |= !isfinite(v);
+    // a warp per column; the FP64 products only where a half of it reaches below the diagonal
+    for (int c = warp; c < d; c += 8) {
+        const double sc = s_scale[c];
+#pragma unroll
+        for (int h = 0; h < 64; h += 32) {
+            const int r = h + lane;
+            T v = T(0);
+            if (h + 31 > c && h < d) v = (T)(A[min(r, d - 1) + c * d] * sc);
+            if (r <= c) v = r == c ? (T)sc : T(0);
+            if (r < d) {
+                out_factor[r + (size_t)c * d] = v;
+                if (out_inverse != nullptr) Lf[r * LDI + c] = (float)v;
+                if (r > c) invalid |= !isfinite(v);
+            }
+        }
     }
     // log|L_jj| in the factor's own precision, summed across lanes then in FP64
     T lg = T(0);

@@ -305,3 +305,37 @@ def test_paired_tiles_density(issm, orc, cuda, form, tol, n, d, k, dof):
             assert np.all(np.abs(a.double().cpu().numpy() - b) <= tol * np.maximum(1.0, np.abs(b)))
         assert int(fail[0].item()) == 0
     issm.ops.check_tensor_core_errors(cuda)
+
+
+# Cholesky backward error, componentwise: |L L^T - A| <= (d + 2) u sqrt(a_ii a_jj),
+# u = eps / 2; l = u_ij / d_j here holds three roundings and the scale sqrt(d) two
+# more: 4 (d + 4) eps. The FP32 inverse is built from products of three levels:
+# |W L - I| <= 4 d eps |W| |L| |W| |L| componentwise.
+@pytest.mark.parametrize("d", [1, 2, 7, 8, 9, 15, 17, 24, 31, 32, 33, 40, 41, 48, 49, 56, 57, 63, 64])
+def test_fit_factor_panels(issm, cuda, d):
+    rng = np.random.default_rng(50 + d)
+    B = rng.normal(size=(d, d)) * 10.0 ** rng.uniform(-3, 3, size=(d, 1))
+    cov = B @ B.T + np.diag(rng.uniform(0.1, 1.0, size=d) * np.diag(B @ B.T))
+    cov = 0.5 * (cov + cov.T)
+    mean, prev = rng.normal(size=d), np.eye(d)
+    scale = np.sqrt(np.outer(np.diag(cov), np.diag(cov)))
+    dp = 16 if d <= 16 else 32 if d <= 32 else 64
+    for dtype, eps in ((torch.float64, 2.0**-52), (torch.float32, 2.0**-23)):
+        loc = torch.empty(d, dtype=dtype, device=cuda)
+        fac = torch.empty(d, d, dtype=dtype, device=cuda)
+        ln = torch.empty(1, dtype=dtype, device=cuda)
+        inv = torch.full((dp, dp), float("nan"), dtype=torch.float32, device=cuda)
+        fail = issm.ops.new_failures(cuda)
+        issm.ops.fit_factor(torch.tensor(mean, device=cuda), torch.tensor(cov, device=cuda),
+                            torch.tensor(prev, device=cuda, dtype=dtype), loc, fac, ln, failures=fail,
+                            regularization=0.0, out_inverse=inv)
+        torch.cuda.synchronize()
+        assert int(fail[0].item()) == 0
+        L = fac.double().cpu().numpy().T
+        assert np.all(np.triu(L, 1) == 0)
+        assert np.all(np.abs(L @ L.T - cov) <= 4 * (d + 4) * eps * scale)
+        W = inv.double().cpu().numpy()
+        assert np.all(W[d:, :] == 0) and np.all(W[:, d:] == 0) and np.all(np.triu(W, 1) == 0)
+        W = W[:d, :d]
+        G = np.abs(W) @ np.abs(L)
+        assert np.all(np.abs(W @ L - np.eye(d)) <= 4 * d * 2.0**-23 * (G @ G))
