@@ -53,14 +53,25 @@ int resample_select(const void *cdf, const void *lw, int64_t n, const void *u, i
 }
 
 // ---- deterministic fixed-point CDF ----------------------------------------------
-__device__ __forceinline__ double det_exp(double x) {
+// e^x 2^bits for x <= 0 (a positive x counts as 0, 0 below -708, NaN passed on). The
+// comparisons, the final scaling and the integer part k of the reduction are
+// integer operations: each FP64 instruction costs a warp 64 cycles of its pipe on
+// this GPU, and these 19 (of 33 with ldexp, floor and FP64 compares) bound the
+// kernels that call it. x >= -708 and 2^-0.5 <= p <= 2^0.5 keep p 2^k normal, so
+// adding to its exponent is exact.
+__device__ __forceinline__ double det_exp(double x, int bits = 0) {
     const double kInvLn2 = 0x1.71547652b82fep+0;
     const double kLn2Hi = 0x1.62e42ff000000p-1;   // ln 2 rounded to 32 bits
     const double kLn2Lo = -0x1.718432a1b0e26p-35; // ln 2 - kLn2Hi
-    if (isnan(x)) return x;
-    if (x < -708.0) return 0.0;
-    if (x > 0.0) x = 0.0;
-    const double k = floor(__dadd_rn(__dmul_rn(x, kInvLn2), 0.5));
+    const long long xb = __double_as_longlong(x);
+    const unsigned long long mag = (unsigned long long)xb & 0x7fffffffffffffffull;
+    if (mag > 0x7ff0000000000000ull) return x;                            // NaN
+    if (xb < 0 && mag > 0x4086200000000000ull) return 0.0;                // x < -708
+    if (xb > 0) x = 0.0;
+    // floor(x / ln 2 + 1/2): rounded down to an integer in the low mantissa bits
+    const double t = __dadd_rd(__dadd_rn(__dmul_rn(x, kInvLn2), 0.5), 0x1.8p52);
+    const int ki = __double2loint(t);
+    const double k = __dadd_rn(t, -0x1.8p52);
     double r = __fma_rn(-k, kLn2Hi, x);
     r = __fma_rn(-k, kLn2Lo, r);
     double p = 1.0 / 6227020800.0;  // 1/13!
@@ -69,7 +80,7 @@ __device__ __forceinline__ double det_exp(double x) {
                                  1.0 / 39916800.0, 1.0 / 479001600.0};
 #pragma unroll
     for (int i = 12; i >= 0; --i) p = __fma_rn(p, r, inv_fact[i]);
-    return ldexp(p, (int)k);
+    return __hiloint2double(__double2hiint(p) + (ki + bits) * (1 << 20), __double2loint(p));
 }
 
 static int fixed_scale_bits(int64_t n) {
@@ -82,10 +93,9 @@ static int fixed_scale_bits(int64_t n) {
 template <typename T> struct FixedWeight {
     const T *lw;
     const double *summary;
-    double scale;
+    int bits;
     __device__ unsigned long long operator()(int64_t i) const {
-        const double w = det_exp(__dadd_rn((double)lw[i], -summary[0]));
-        return (unsigned long long)floor(__dadd_rn(__dmul_rn(w, scale), 0.5));
+        return __double2ull_rd(__dadd_rn(det_exp(__dadd_rn((double)lw[i], -summary[0]), bits), 0.5));
     }
 };
 
@@ -142,14 +152,14 @@ int resample_fixed(const void *lw, int64_t n, int dtype, const double *uniforms,
     unsigned long long *tiles = prefix + (n + 1);
     int st = logweight_summary(lw, n, dtype, summary, base, red, stream);
     if (st) return st;
-    const double scale = ldexp(1.0, fixed_scale_bits(n));
+    const int bits = fixed_scale_bits(n);
     // a fixed-point weight is some twenty FP64 operations on this GPU's narrow
     // FP64 pipe: formed once, kept where its prefix will go
     if (dtype == ISSM_F32)
-        st = scan_apply_kept<unsigned long long>(n, FixedWeight<float>{(const float *)lw, summary, scale},
+        st = scan_apply_kept<unsigned long long>(n, FixedWeight<float>{(const float *)lw, summary, bits},
                                                  PrefixWrite{prefix}, tiles, prefix, stream);
     else
-        st = scan_apply_kept<unsigned long long>(n, FixedWeight<double>{(const double *)lw, summary, scale},
+        st = scan_apply_kept<unsigned long long>(n, FixedWeight<double>{(const double *)lw, summary, bits},
                                                  PrefixWrite{prefix}, tiles, prefix, stream);
     if (st) return st;
     if (count <= 0) return 0;
