@@ -11,6 +11,7 @@
 #include <cmath>
 
 #include "../../include/issm.h"
+#include "dmath.cuh"
 
 namespace issm {
 
@@ -80,13 +81,30 @@ template <typename T> struct LseState {
     T s = T(0);
     bool nan = false;
     __device__ __forceinline__ void add(T t) {
+        if constexpr (sizeof(T) == 8) {
+            // comparisons by the bits, one FMA for both updates: FP64 instructions are what this costs
+            const uint32_t hi = (uint32_t)__double2hiint(t), lo = (uint32_t)__double2loint(t);
+            const uint32_t mag = hi & 0x7fffffffu;
+            if (mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0)) {
+                nan = true;
+            } else if (hi != 0xfff00000u) {  // not -Inf
+                const bool up = t > m;
+                const T gap = up ? m - t : t - m;  // <= 0; NaN for equal infinities
+                const uint32_t g = (uint32_t)__double2hiint(gap) & 0x7fffffffu;
+                // beyond 37.5 a term is below half an ulp of the sum; equal infinities count as equal
+                T e = g < 0x4042c000u ? table_exp(gap) : t == m ? T(1) : T(0);
+                s = fma(up ? s : e, up ? e : T(1), up ? T(1) : s);
+                m = up ? t : m;
+            }
+            return;
+        }
         if (isnan(t)) {
             nan = true;
         } else if (t > -num<T>::inf()) {
             const bool up = t > m;
             const T gap = up ? m - t : t - m;  // <= 0; NaN for equal infinities
             T e = t == m ? T(1) : T(0);
-            if (sizeof(T) == 4 ? t != m : gap > (up ? T(-60) : T(-37.5)) && t != m) e = dexp(gap);
+            if (t != m) e = dexp(gap);
             s = up ? s * e + T(1) : s + e;
             m = up ? t : m;
         }

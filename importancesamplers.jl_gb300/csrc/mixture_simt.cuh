@@ -381,10 +381,22 @@ __device__ __forceinline__ void factor_radius(const T *__restrict__ c, const T (
 template <typename T>
 __device__ __forceinline__ T radial_logdensity(const T *__restrict__ c, T r2, int family, bool *slow) {
     if (family == ISSM_GAUSSIAN) {
-        if (!isfinite(r2)) { *slow = true; return T(0); }
+        bool finite;
+        if constexpr (sizeof(T) == 8) finite = (__double2hiint(r2) & 0x7ff00000) != 0x7ff00000;  // no FP64 instruction
+        else finite = isfinite(r2);
+        if (!finite) { *slow = true; return T(0); }
         return c[0] - T(0.5) * r2;
     }
     const T ratio = quotient(r2, c[2], c[4]);
+    if constexpr (sizeof(T) == 8) {
+        // c[3] is 0 or 1; r2 >= 0 or NaN: its order is its bits'
+        const uint32_t b = (uint32_t)__double2hiint(r2), q = (uint32_t)__double2hiint(ratio);
+        if (__double2hiint(c[3]) != 0 || b < 0x00100000u || b >= 0x7ff00000u || q >= 0x7ff00000u) {
+            *slow = true;
+            return T(0);
+        }
+        return c[0] - c[5] * table_log1p(ratio);
+    }
     if (c[3] != T(0) || r2 < num<T>::fmin() || !isfinite(ratio)) { *slow = true; return T(0); }
     return c[0] - c[5] * dlog1p(ratio);
 }

@@ -339,3 +339,46 @@ def test_fit_factor_panels(issm, cuda, d):
         W = W[:d, :d]
         G = np.abs(W) @ np.abs(L)
         assert np.all(np.abs(W @ L - np.eye(d)) <= 4 * d * 2.0**-23 * (G @ G))
+
+
+# The FP64 component density in one dimension, L = 1, mu = 0: the ratio x^2 / nu
+# holds at most two roundings (2 eps of it, log1p's condition is below 1), log1p 1.5
+# ulp, the final product and sum one each: 5 eps of |c| + (nu + 1) / 2 log1p covers it.
+@pytest.mark.parametrize("dof", [1.0, 3.0, 1e6])
+def test_f64_student_radius_range(issm, cuda, dof):
+    """Ratios from 0 and the subnormals through every table interval and its edges
+    to the largest finite ones."""
+    rng = np.random.default_rng(3)
+    j = np.arange(-4, 260)
+    edges = np.concatenate([np.ldexp(1.0 + np.clip(j, 0, 255) / 128.0, e) - 1.0 for e in (0, 1, 7, 52, 53, 60)])
+    edges = np.concatenate([np.nextafter(edges, 0), edges, np.nextafter(edges, np.inf)])
+    wide = np.exp(rng.uniform(np.log(1e-290), np.log(1e290), size=4096))
+    ratio = np.concatenate([[0.0, 2.0**-53, 2.0**-52, 0.5, 1.0], np.abs(edges), wide])
+    x = np.sqrt(ratio * dof)
+    one = np.ones((1, 1))
+    db = issm.pack_proposals([issm.FactorStudentT(np.float64(dof), np.zeros(1), one)], cuda)
+    den = issm.ops.denominator(issm.native.DENOM_FULL, torch.zeros(1, device=cuda, dtype=torch.float64))
+    got = issm.ops.mixture_logdensity(db, den, torch.tensor(x[:, None], device=cuda)).cpu().numpy()
+    c = float(db.lognormalizers[0].item())
+    xl = x.astype(np.longdouble)
+    radial = (np.longdouble(dof + 1.0) / 2.0 * np.log1p(xl * xl / dof)).astype(np.float64)
+    assert np.all(np.abs(got - (c - radial)) <= 5 * 2.0**-52 * (abs(c) + radial))
+
+
+# A log-sum-exp of K terms: each exponential 0.51 ulp plus its argument's rounding
+# (half an ulp of a gap below 37.5: 2^-48 of the term, 64 eps / 4), each sum one rounding;
+# (16 + K) eps of the sum and 2 eps of the value.
+@pytest.mark.parametrize("k", [2, 5, 40, 130])
+def test_f64_log_sum_exp(issm, cuda, k):
+    rng = np.random.default_rng(k)
+    db = issm.pack_proposals([issm.FactorGaussian(np.zeros(2), np.eye(2)) for _ in range(k)], cuda)
+    x = rng.normal(size=(700, 2))
+    for coef in (np.zeros(k), -40.0 * rng.random(k), -np.arange(k) * np.log(2.0) / 128.0,
+                 np.where(np.arange(k) % 3 == 1, -np.inf, -800.0 * rng.random(k))):
+        den = issm.ops.denominator(issm.native.DENOM_FULL, torch.tensor(coef, device=cuda))
+        got = issm.ops.mixture_logdensity(db, den, torch.tensor(x, device=cuda)).cpu().numpy()
+        xl = x.astype(np.longdouble)
+        lq = -np.log(2 * np.longdouble(np.pi)) - 0.5 * (xl * xl).sum(1)
+        m = coef.max()
+        want = (lq + m + np.log(np.exp((coef - m).astype(np.longdouble)).sum())).astype(np.float64)
+        assert np.all(np.abs(got - want) <= 2.0**-52 * (16 + k + 4 * (np.abs(want) + abs(m) + np.abs(lq.astype(np.float64)))))
