@@ -34,6 +34,11 @@ int normalize(const void *lw, int64_t n, int dtype, const double *summary, void 
 int amis_form_summary(const void *lt, const void *lnum, const int64_t *round_ids, double logtotal, int64_t n,
                       int dtype, void *lw, uint64_t *failures, double *out, void *ws, size_t ws_bytes,
                       cudaStream_t stream);
+// the same with the targets of samples first_new.. checked in the pass (an invalid
+// one leaves the round); the workspace's first word is zero, and is again afterwards
+int amis_round_summary(const void *lt, const void *lnum, int64_t *round_ids, double logtotal, int64_t n,
+                       int64_t first_new, int dtype, void *lw, uint64_t *failures, double *out, void *ws,
+                       size_t ws_bytes, cudaStream_t stream);
 int resampling_cdf(const void *lw, int64_t n, int dtype, void *cdf, void *ws, size_t ws_bytes,
                    cudaStream_t stream);
 
@@ -55,7 +60,8 @@ int weighted_moments(const void *x, int d, int64_t n, const void *lw, int dtype,
                      cudaStream_t stream);
 int fit_factor(const double *mean, const double *cov, int d, const void *prev, double dof, double logconst,
                int dtype, void *out_loc, void *out_factor, void *out_lognorm, uint64_t *failures,
-               int64_t failure_index, float *out_inverse, double regularization, cudaStream_t stream);
+               int64_t failure_index, float *out_inverse, double regularization, cudaStream_t stream,
+               double *out_shift = nullptr);
 
 // population local weights, covariances, factors (population.cu)
 int population_local_weights(const void *lw, const void *x, int d, int dtype, const int64_t *starts,

@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(256) fit_factor_kernel(const double *__restric
                                                          double ridge_fallback_scale, double lognorm_const,
                                                          double tscale, T *out_loc, T *out_factor, T *out_lognorm,
                                                          uint64_t *failures, int64_t failure_index,
-                                                         float *out_inverse) {
+                                                         float *out_inverse, double *out_shift) {
     extern __shared__ __align__(16) double A[];  // d x d column-major
     __shared__ double s_red[8];
     __shared__ double s_ridge;
@@ -405,6 +405,7 @@ __global__ void __launch_bounds__(256) fit_factor_kernel(const double *__restric
     for (int c = tid; c < d; c += 256) {
         const T v = (T)mean[c];
         out_loc[c] = v;
+        if (out_shift != nullptr) out_shift[c] = (double)v;
         invalid |= !isfinite(v);
     }
     lg = warp_sum_all(lg);
@@ -434,7 +435,8 @@ __global__ void __launch_bounds__(256) fit_factor_kernel(const double *__restric
 
 int fit_factor(const double *mean, const double *cov, int d, const void *prev, double dof, double logconst,
                int dtype, void *out_loc, void *out_factor, void *out_lognorm, uint64_t *failures,
-               int64_t failure_index, float *out_inverse, double regularization, cudaStream_t stream) {
+               int64_t failure_index, float *out_inverse, double regularization, cudaStream_t stream,
+               double *out_shift) {
     if (d > 64) return ISSM_E_UNSUPPORTED;
     size_t smem = sizeof(double) * (size_t)d * d;
     if (out_inverse != nullptr) {
@@ -456,13 +458,13 @@ int fit_factor(const double *mean, const double *cov, int d, const void *prev, d
         { fit_factor_kernel<float><<<1, 256, smem, stream>>>(mean, cov, d, (const float *)prev, ridge_scale,
                                                            ridge_fallback, lognorm_const, tscale, (float *)out_loc,
                                                            (float *)out_factor, (float *)out_lognorm, failures,
-                                                           failure_index, out_inverse); note_launch(); }
+                                                           failure_index, out_inverse, out_shift); note_launch(); }
     } else {
         { fit_factor_kernel<double><<<1, 256, smem, stream>>>(mean, cov, d, (const double *)prev, ridge_scale,
                                                             ridge_fallback, lognorm_const, tscale,
                                                             (double *)out_loc, (double *)out_factor,
                                                             (double *)out_lognorm, failures, failure_index,
-                                                            out_inverse); note_launch(); }
+                                                            out_inverse, out_shift); note_launch(); }
     }
     return (int)cudaGetLastError();
 }

@@ -139,6 +139,7 @@ __device__ void summary_finish(const ThreadSums<double> &ts, double *out, Moment
     __syncthreads();
     if (!last) return;
     __threadfence();
+    if (threadIdx.x == 0) *counter = 0u;  // every CTA has counted: ready for the next launch
     // the last block merges the per-block partials the same way
     const volatile double *pv = reinterpret_cast<const volatile double *>(partials);
     double pm = -INFINITY, ps = 0.0, ps2 = 0.0;
@@ -245,6 +246,7 @@ __device__ void summary_finish(const ThreadSums<float> &ts, double *out, Moments
     __syncthreads();
     if (!last) return;
     __threadfence();
+    if (threadIdx.x == 0) *counter = 0u;  // every CTA has counted: ready for the next launch
     // the last block: this thread's partials about their own maximum, then the block merge
     const volatile float *pv = reinterpret_cast<const volatile float *>(partials);
     constexpr int kW = sizeof(Partial3f) / sizeof(float);
@@ -297,17 +299,27 @@ __global__ void __launch_bounds__(256) summary_kernel(const T *__restrict__ lw, 
 // (_form_amis_logweights_kernel!, src/amis_execution.jl:107-134, then
 // _logweight_summary): logw_i = logtarget_i - (lognum_i - logtotal) for
 // round_ids[i] != 0, recording invalid weights; only the weights written
-// enter the summary.
+// enter the summary. The targets of samples from first_new on are checked here
+// as check_targets_kernel does (indices from the first new sample): an invalid
+// one is recorded and its round id becomes 0.
 template <typename T>
 __global__ void __launch_bounds__(256) form_summary_kernel(const T *__restrict__ lt, const T *__restrict__ lnum,
-                                                           const int64_t *__restrict__ round_ids, T logtotal,
-                                                           int64_t n, T *__restrict__ lw, uint64_t *failures,
+                                                           int64_t *round_ids, T logtotal, int64_t n,
+                                                           int64_t first_new, T *__restrict__ lw, uint64_t *failures,
                                                            double *out, Moments3 *partials, unsigned int *counter) {
     ThreadSums<T> ts;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     auto one = [&](int64_t i, T target, T num) {
         T v;
+        if (i >= first_new) {
+            const uint16_t reason = target_reason(target);
+            if (reason) {
+                record_failure(failures, i - first_new + 1, 0, reason);
+                if (round_ids) round_ids[i] = 0;
+                return;
+            }
+        }
         const uint16_t r = subtract_logweight(target, num - logtotal, &v);
         if (r) {
             record_failure(failures, i + 1, 0, r);
@@ -385,24 +397,33 @@ int logweight_summary(const void *lw, int64_t n, int dtype, double *out, void *w
     return summary_launch(lw, n, dtype, out, ws, stream);
 }
 
+int amis_round_summary(const void *lt, const void *lnum, int64_t *round_ids, double logtotal, int64_t n,
+                       int64_t first_new, int dtype, void *lw, uint64_t *failures, double *out, void *ws,
+                       size_t ws_bytes, cudaStream_t stream) {
+    if (ws_bytes < reduce_workspace_bytes(n)) return ISSM_E_WORKSPACE;
+    unsigned int *counter = (unsigned int *)ws;
+    Moments3 *partials = (Moments3 *)((char *)ws + 256);
+    const int blocks = summary_blocks(n, dtype);
+    if (dtype == ISSM_F32)
+        { form_summary_kernel<float><<<blocks, 256, 0, stream>>>((const float *)lt, (const float *)lnum, round_ids,
+                                                               (float)logtotal, n, first_new, (float *)lw, failures,
+                                                               out, partials, counter); note_launch(); }
+    else
+        { form_summary_kernel<double><<<blocks, 256, 0, stream>>>((const double *)lt, (const double *)lnum,
+                                                                round_ids, logtotal, n, first_new, (double *)lw,
+                                                                failures, out, partials, counter); note_launch(); }
+    return (int)cudaGetLastError();
+}
+
 int amis_form_summary(const void *lt, const void *lnum, const int64_t *round_ids, double logtotal, int64_t n,
                       int dtype, void *lw, uint64_t *failures, double *out, void *ws, size_t ws_bytes,
                       cudaStream_t stream) {
     if (ws_bytes < reduce_workspace_bytes(n)) return ISSM_E_WORKSPACE;
-    unsigned int *counter = (unsigned int *)ws;
-    Moments3 *partials = (Moments3 *)((char *)ws + 256);
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream);
+    cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(unsigned int), stream);
     if (e != cudaSuccess) return (int)e;
-    const int blocks = summary_blocks(n, dtype);
-    if (dtype == ISSM_F32)
-        { form_summary_kernel<float><<<blocks, 256, 0, stream>>>((const float *)lt, (const float *)lnum, round_ids,
-                                                               (float)logtotal, n, (float *)lw, failures, out,
-                                                               partials, counter); note_launch(); }
-    else
-        { form_summary_kernel<double><<<blocks, 256, 0, stream>>>((const double *)lt, (const double *)lnum,
-                                                                round_ids, logtotal, n, (double *)lw, failures,
-                                                                out, partials, counter); note_launch(); }
-    return (int)cudaGetLastError();
+    // no sample is new: nothing is checked and no round id written
+    return amis_round_summary(lt, lnum, const_cast<int64_t *>(round_ids), logtotal, n, n, dtype, lw, failures, out, ws,
+                              ws_bytes, stream);
 }
 
 template <typename T>

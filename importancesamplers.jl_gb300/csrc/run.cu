@@ -1,9 +1,12 @@
 // run.cu — one AMIS run issued from native code: every launch of every
 // round, stream-ordered, no host synchronisation, in one C call. It performs
-// the same sequence of library calls as the Python round loop
-// (sampler.py::_moment_body), so its results are bitwise the same; the point
-// is the host cost: one call instead of a dozen interpreted calls per round,
-// which is what bounds a serving loop of many small runs.
+// the same computations as the Python round loop (sampler.py::_moment_body), so
+// its results are bitwise the same; the point is the host cost: one call instead
+// of a dozen interpreted calls per round, which is what bounds a serving loop of
+// many small runs. Small rounds are bound by their chain of launches, about 2.3
+// us each with the gap: the targets' check rides in the weights' pass, the fit
+// leaves the next round's shift in FP64 and the summary its counter at zero, three
+// launches fewer a round.
 //
 // Reference counterpart: one AMIS round (_launch_prefilled_amis_round!,
 // src/amis_execution.jl:261-357: draw, target, retrospective append, prefix
@@ -120,8 +123,6 @@ int issm_amis_run(const issm_amis_run_desc *r, issm_stream_t stream) {
                                          (int32_t *)(ws_tc + tc_bytes - 64), stream));
         else
             ISSM_TRY(issm_target_logdensity(r->target, x_new, n_new, logtargets + (size_t)n_old * es, stream));
-        ISSM_TRY(issm_check_target_values(logtargets + (size_t)n_old * es, n_new, h.dtype, r->round_ids + n_old, fail,
-                                          0, stream));
         // retrospective append over the retained samples, then the prefix mixture of the new ones
         if (n_old > 0) {
             if (tc)
@@ -138,16 +139,20 @@ int issm_amis_run(const issm_amis_run_desc *r, issm_stream_t stream) {
             ISSM_TRY(issm_mixture_logdensity(&view, &den, x_new, n_new, nullptr, t, lognum + (size_t)n_old * es, nullptr,
                                              fail, 0, r->precision, stream));
         double *summary = r->summaries + 3 * t;
-        ISSM_TRY(issm_amis_form_summary(logtargets, lognum, r->round_ids, std::log((double)n_tot), n_tot, h.dtype,
-                                        r->logweights, fail, summary, ws_red, red_bytes, stream));
-        // moments about the previous location, then the FP64 fit into slot t + 1 (or the candidate)
-        if (h.dtype == ISSM_F32) {
-            to_f64_kernel<float><<<1, 64, 0, s>>>((const float *)(loc + (size_t)t * d * es), d, r->shift);
-        } else {
-            to_f64_kernel<double><<<1, 64, 0, s>>>((const double *)(loc + (size_t)t * d * es), d, r->shift);
+        // the new samples' targets are checked in the same pass
+        ISSM_TRY(amis_round_summary(logtargets, lognum, r->round_ids, std::log((double)n_tot), n_tot, n_old, h.dtype,
+                                    r->logweights, fail, summary, ws_red, red_bytes, s));
+        // moments about the previous location (kept in FP64 by the fit that wrote
+        // it), then the FP64 fit into slot t + 1 (or the candidate)
+        if (t == 0) {
+            if (h.dtype == ISSM_F32) {
+                to_f64_kernel<float><<<1, 64, 0, s>>>((const float *)loc, d, r->shift);
+            } else {
+                to_f64_kernel<double><<<1, 64, 0, s>>>((const double *)loc, d, r->shift);
+            }
+            note_launch();
+            ISSM_TRY((int)cudaGetLastError());
         }
-        note_launch();
-        ISSM_TRY((int)cudaGetLastError());
         const void *prev = fac + (size_t)t * d * d * es;
         ISSM_TRY(issm_weighted_moments_ws(samples, d, n_tot, r->logweights, h.dtype, summary, r->shift,
                                           h.dtype == ISSM_F32 ? prev : nullptr, r->mean, r->cov, r->precision, ws_mom,
@@ -157,8 +162,8 @@ int issm_amis_run(const issm_amis_run_desc *r, issm_stream_t stream) {
         void *out_fac = last ? r->cand_factor : (void *)(fac + (size_t)(t + 1) * d * d * es);
         void *out_ln = last ? r->cand_lognormalizer : (void *)(lnorm + (size_t)(t + 1) * es);
         float *out_inv = (!last && tc) ? (float *)h.inverse_factors + (size_t)(t + 1) * dp * dp : nullptr;
-        ISSM_TRY(issm_fit_factor_ex(r->mean, r->cov, d, prev, 0.0, r->logconstant, h.dtype, out_loc, out_fac, out_ln,
-                                    out_inv, fail, n_tot + 1, stream));
+        ISSM_TRY(fit_factor(r->mean, r->cov, d, prev, 0.0, r->logconstant, h.dtype, out_loc, out_fac, out_ln, fail,
+                            n_tot + 1, out_inv, -1.0, s, last ? nullptr : r->shift));
         n_old = n_tot;
     }
     if (r->counter) ISSM_TRY(issm_counter_advance(r->counter, offset - r->normal_offset, stream));

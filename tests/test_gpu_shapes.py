@@ -382,3 +382,23 @@ def test_f64_log_sum_exp(issm, cuda, k):
         m = coef.max()
         want = (lq + m + np.log(np.exp((coef - m).astype(np.longdouble)).sum())).astype(np.float64)
         assert np.all(np.abs(got - want) <= 2.0**-52 * (16 + k + 4 * (np.abs(want) + abs(m) + np.abs(lq.astype(np.float64)))))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("size", [1, 3, 500, 4099])
+def test_round_summary_checks_new_targets(issm, cuda, dtype, size):
+    """Invalid targets recorded by the weights' pass of a native run: the failure
+    words, round ids and summaries of the separate check."""
+    d = 2
+    target = issm.QuadraticTarget(np.zeros(d), float("nan"))
+    p = issm.FactorGaussian(np.zeros(d, dtype=dtype), np.eye(d, dtype=dtype))
+    out = []
+    for body in (issm.sampler._native_body, lambda s: issm.sampler._moment_body(s, False)):
+        s = issm.prepare_sampler(3, target, issm.AMIS(p, rounds=3, round_size=size), device=cuda, graphs=False)
+        body(s)
+        torch.cuda.synchronize()
+        out.append((s.round_failures.cpu(), s.round_ids.cpu(), s.summaries[0].cpu()))
+    assert int(out[0][0][0, 0]) >= size and int(out[0][1].abs().sum()) == 0
+    for a, b in zip(*out):
+        assert torch.equal(a.nan_to_num(nan=-1.0) if a.is_floating_point() else a,
+                           b.nan_to_num(nan=-1.0) if b.is_floating_point() else b)
