@@ -12,32 +12,32 @@
 //     chunk is one bulk copy: 37% fewer bytes and MMA columns at DP = 64;
 //   * the offset -b_k is one K slice of the hi parts alone, two operand columns
 //     hi(-b) and lo(-b) against samples extended by (1, 1).
-// One CTA per SM walks pairs of tiles:
+// One CTA per SM walks pairs of tiles; an item is a (pair, chunk):
 //   warps 1-8   read the next pair's rows into registers, centre, round and
 //               split them into the A operand (two tiles, one buffer);
-//   warp 0      copies the chunks through a ring of three slots and issues item
-//               j's (pair, chunk) MMAs into one of two accumulator pairs;
+//   warps 0, 17 issue the MMAs of the even and the odd items, each into its own
+//               pair of accumulators;
+//   warp 18     copies the chunks through a ring of four slots;
 //   warps 9-16  reduce the other: four warps (TMEM lane quadrants) per tile,
 //               |z|^2 per component, the radial density and an online
 //               log-sum-exp that takes a chunk's terms at once.
 // One tile at a time, full operand squares and one epilogue warp per quadrant
 // ran at 33 bytes of operands per clock and SM out of L2, 1,268 us for
-// 1,000,003 samples x 40 components, d = 64 (BF16x3); this form takes 769 us, and
-// 1,139 against 3,766 us for 4,194,304 x 64, d = 16. Tensor time is 1,418 clocks
-// per (pair, chunk) of d = 64, about 370 us of the 769; the epilogue's TMEM reads and
-// the handover between the two bound the rest. Few samples share the tiles out
-// worse (pairs, not tiles, per SM), yet 50,000 x 40, d = 64 still gains: 91 to
-// 79 us; x 8 is even at 35.5. Every wait is bounded; a
-// timeout sets the sticky error word and the CTA unwinds after draining its
-// copies and MMAs.
+// 1,000,003 samples x 40 components, d = 64 (BF16x3); this form takes 497, 370 of
+// them tensor time (1,418 clocks per item). 4,194,304 x 64, d = 16: 3,766 -> 1,095,
+// bound by the epilogue's exponentials. Few samples share the tiles out worse
+// (pairs, not tiles, per SM), yet 50,000 x 40, d = 64 still gains, 91 -> 58, and
+// x 8 35.5 -> 31.4. Every wait is bounded; a timeout sets the sticky error word and
+// the CTA unwinds after draining its copies and MMAs.
 #include "mixture_tc.cuh"
 
 namespace issm {
 
 constexpr int kPairConvWarps = 8, kPairEpiWarps = 8;
 constexpr int kPairFirstEpi = 1 + kPairConvWarps;
-constexpr int kPairThreads = 32 * (1 + kPairConvWarps + kPairEpiWarps);
-constexpr int kPairRing = 3;
+constexpr int kPairIssuer2 = kPairFirstEpi + kPairEpiWarps, kPairLoader = kPairIssuer2 + 1;
+constexpr int kPairThreads = 32 * (kPairLoader + 1);
+constexpr int kPairRing = 4;  // even: a slot's items are one issuer's
 constexpr int kPairN = 128;  // accumulator columns of one tile: operand rows of a chunk
 
 template <int KIND, int SPLIT, int DP> struct PairShape {
@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) mixture_pair_kernel(TcParams 
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *s_a = smem;                // two tiles
     unsigned char *s_b = smem + 2 * S::TILE;  // ring of chunks
-    __shared__ __align__(8) uint64_t a_full, a_empty, b_full[kPairRing], b_empty[kPairRing], d_full[2], d_empty[2];
+    __shared__ __align__(8) uint64_t a_full, a_empty, b_full[kPairRing], b_empty[kPairRing], d_full[2], d_empty[2],
+        drained[2];
     __shared__ __align__(16) float s_c[DP];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int abort_flag;
@@ -128,8 +129,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) mixture_pair_kernel(TcParams 
     if (warp == 0) tc::tmem_alloc(&tmem_base, 512);
     if (tid == 0) {
         tc::mbar_init(&a_full, kPairConvWarps);
-        tc::mbar_init(&a_empty, 1);
+        tc::mbar_init(&a_empty, 2);
         for (int b = 0; b < 2; ++b) {
+            tc::mbar_init(&drained[b], 1);
             tc::mbar_init(&d_full[b], 1);
             tc::mbar_init(&d_empty[b], kPairEpiWarps);
         }
@@ -167,83 +169,87 @@ __global__ void __launch_bounds__(kPairThreads, 1) mixture_pair_kernel(TcParams 
     const int J = my_pairs * nchunks;
     auto row0_of = [&](int it) -> int64_t { return ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * (2 * kTcTile); };
 
-    if (warp == 0) {
-        // ================= issuer: chunks in, MMAs out =================
-        int issued = 0, waited = 0, ch_load = 0;
-        auto load = [&]() {
-            const int slot = issued % kPairRing;
-            if (lane == 0) {
-                tc::mbar_arrive_expect_tx(&b_full[slot], S::CHUNK);
-                tc::bulk_copy_g2s(s_b + (size_t)slot * S::CHUNK, p.ops + (size_t)ch_load * S::CHUNK, S::CHUNK, &b_full[slot]);
-            }
-            __syncwarp();
-            ++issued;
-            if (++ch_load == nchunks) ch_load = 0;
-        };
-        for (int q = 0; q < kPairRing && q < J; ++q) load();
-        int ok = 1, it = 0, ch = 0;
-        for (int j = 0; j < J && ok; ++j) {
+    if (warp == 0 || warp == kPairIssuer2) {
+        // ================= issuers: warp 0 the even items, warp 17 the odd ones =================
+        // An issuer's waits before its next item run while the other's MMAs do: one
+        // issuer, blocked while its MMAs queue and then waiting on four barriers, took
+        // 2,790 clocks per item (764 us in all), two take 1,815 (497). Items alternate accumulator pairs and, the ring being even,
+        // slots, so an issuer sees every phase of the barriers it waits on.
+        const int mine = warp == 0 ? 0 : 1;
+        int it = 0, ch = mine, seen = -1;
+        for (int j = mine; j < J; j += 2) {
             const int slot = j % kPairRing;
-            {
-                bool fine = ch != 0 || wait(&a_full, (uint32_t)(it & 1));
-                if (fine) fine = wait(&b_full[slot], (uint32_t)((j / kPairRing) & 1));
-                if (fine) waited = j + 1;
-                if (fine && j >= 2) fine = wait(&d_empty[j & 1], (uint32_t)(((j - 2) >> 1) & 1));
-                fine = __all_sync(0xffffffffu, fine);
-                tc::fence_after_sync();
-                if (fine) {
-                    const uint32_t b0 = tc::smem_u32(s_b + (size_t)slot * S::CHUNK);
-                    const uint32_t full = tc::instr_desc(KIND, kTcTile, kPairN);
-                    const uint64_t db0 = tc::smem_desc(b0, S::GROUP, 128);
+            bool fine = seen == it || wait(&a_full, (uint32_t)(it & 1));
+            seen = it;
+            if (fine) fine = wait(&b_full[slot], (uint32_t)((j / kPairRing) & 1));
+            if (fine && j >= 2) fine = wait(&d_empty[mine], (uint32_t)(((j - 2) >> 1) & 1));
+            fine = __all_sync(0xffffffffu, fine);
+            tc::fence_after_sync();
+            if (fine) {
+                const uint32_t b0 = tc::smem_u32(s_b + (size_t)slot * S::CHUNK);
+                const uint32_t full = tc::instr_desc(KIND, kTcTile, kPairN);
+                const uint64_t db0 = tc::smem_desc(b0, S::GROUP, 128);
 #pragma unroll
-                    for (int g = 0; g < 2; ++g) {
-                        const uint32_t a0 = tc::smem_u32(s_a + g * S::TILE);
-                        const uint32_t dt = tbase + (uint32_t)((j & 1) * 2 * kPairN + g * kPairN);
-                        const uint64_t da0 = tc::smem_desc(a0 + S::KG * S::GROUP, S::GROUP, 128);
-                        if (KIND == tc::kTF32) tc::mma_tf32_elect(dt, da0, db0, full, false);
-                        else tc::mma_elect(dt, da0, db0, full, false);
+                for (int g = 0; g < 2; ++g) {
+                    const uint32_t a0 = tc::smem_u32(s_a + g * S::TILE);
+                    const uint32_t dt = tbase + (uint32_t)(mine * 2 * kPairN + g * kPairN);
+                    const uint64_t da0 = tc::smem_desc(a0 + S::KG * S::GROUP, S::GROUP, 128);
+                    if (KIND == tc::kTF32) tc::mma_tf32_elect(dt, da0, db0, full, false);
+                    else tc::mma_elect(dt, da0, db0, full, false);
 #pragma unroll
-                        for (int s = 0; s < S::KSTEPS; ++s) {
-                            // operand rows j >= 2 PER s: the last columns of the accumulator
-                            const int n0 = S::first(s);
-                            const uint32_t lbo = (uint32_t)(kPairN - n0) * 16;
-                            const uint32_t idesc = tc::instr_desc(KIND, kTcTile, kPairN - n0);
-                            const uint64_t da = tc::smem_desc(a0 + s * 2 * S::GROUP, S::GROUP, 128);
-                            const uint64_t db = tc::smem_desc(b0 + S::slice(0, s), lbo, 128);
-                            if (KIND == tc::kTF32) {
-                                tc::mma_tf32_elect(dt + n0, da, db, idesc, true);
-                            } else {
-                                tc::mma_elect(dt + n0, da, db, idesc, true);
-                                if (SPLIT == 3) {
-                                    const uint64_t dal = tc::smem_desc(a0 + (S::KGX + s * 2) * S::GROUP, S::GROUP, 128);
-                                    const uint64_t dbl = tc::smem_desc(b0 + S::slice(1, s), lbo, 128);
-                                    tc::mma_elect(dt + n0, dal, db, idesc, true);
-                                    tc::mma_elect(dt + n0, da, dbl, idesc, true);
-                                }
+                    for (int s = 0; s < S::KSTEPS; ++s) {
+                        // operand rows j >= 2 PER s: the last columns of the accumulator
+                        const int n0 = S::first(s);
+                        const uint32_t lbo = (uint32_t)(kPairN - n0) * 16;
+                        const uint32_t idesc = tc::instr_desc(KIND, kTcTile, kPairN - n0);
+                        const uint64_t da = tc::smem_desc(a0 + s * 2 * S::GROUP, S::GROUP, 128);
+                        const uint64_t db = tc::smem_desc(b0 + S::slice(0, s), lbo, 128);
+                        if (KIND == tc::kTF32) {
+                            tc::mma_tf32_elect(dt + n0, da, db, idesc, true);
+                        } else {
+                            tc::mma_elect(dt + n0, da, db, idesc, true);
+                            if (SPLIT == 3) {
+                                const uint64_t dal = tc::smem_desc(a0 + (S::KGX + s * 2) * S::GROUP, S::GROUP, 128);
+                                const uint64_t dbl = tc::smem_desc(b0 + S::slice(1, s), lbo, 128);
+                                tc::mma_elect(dt + n0, dal, db, idesc, true);
+                                tc::mma_elect(dt + n0, da, dbl, idesc, true);
                             }
                         }
                     }
                 }
-                // commits arrive when every earlier MMA has completed, issued or not
-                tc::commit_elect(&d_full[j & 1]);
-                tc::commit_elect(&b_empty[slot]);
-                if (ch == nchunks - 1) tc::commit_elect(&a_empty);
-                if (!fine) ok = 0;
             }
-            // refill the slot the previous item's MMAs have finished with
-            if (ok && j >= 1 && j + kPairRing - 1 < J) {
-                int fine = 1;
-                if (lane == 0) fine = wait(&b_empty[(j - 1) % kPairRing], (uint32_t)(((j - 1) / kPairRing) & 1));
-                if (__shfl_sync(0xffffffffu, fine, 0)) load();
-            }
-            if (++ch == nchunks) {
-                ch = 0;
+            // commits arrive when this issuer's earlier MMAs have completed, issued or not
+            tc::commit_elect(&d_full[mine]);
+            tc::commit_elect(&b_empty[slot]);
+            if (ch + 2 >= nchunks) tc::commit_elect(&a_empty);  // my last item of the pair
+            if (!fine) break;
+            ch += 2;
+            if (ch >= nchunks) {
+                ch -= nchunks;
                 ++it;
             }
         }
+        // drain: my MMAs have completed before the accumulators are freed
+        tc::commit_elect(&drained[mine]);
+        tc::mbar_wait(&drained[mine], 0u);
+    } else if (warp == kPairLoader) {
+        // ================= loader: chunks into the ring =================
+        int issued = 0, ch = 0;
+        for (int j = 0; j < J; ++j) {
+            const int slot = j % kPairRing;
+            if (j >= kPairRing && !__all_sync(0xffffffffu, wait(&b_empty[slot], (uint32_t)((j / kPairRing - 1) & 1)))) break;
+            if (lane == 0) {
+                tc::mbar_arrive_expect_tx(&b_full[slot], S::CHUNK);
+                tc::bulk_copy_g2s(s_b + (size_t)slot * S::CHUNK, p.ops + (size_t)ch * S::CHUNK, S::CHUNK, &b_full[slot]);
+            }
+            __syncwarp();
+            issued = j + 1;
+            if (++ch == nchunks) ch = 0;
+        }
         // drain: every requested copy has landed before the CTA exits
         if (lane == 0)
-            for (int q = waited; q < issued; ++q) tc::mbar_wait(&b_full[q % kPairRing], (uint32_t)((q / kPairRing) & 1));
+            for (int q = max(0, issued - kPairRing); q < issued; ++q)
+                tc::mbar_wait(&b_full[q % kPairRing], (uint32_t)((q / kPairRing) & 1));
     } else if (warp < kPairFirstEpi) {
         // ================= converters: half a row of each tile per thread =================
         const int ctid = tid - 32, row = ctid & (kTcTile - 1), half = ctid >> 7;
@@ -378,8 +384,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) mixture_pair_kernel(TcParams 
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (tid == 0 && abort_flag && J > 0) tc::mbar_wait(&d_full[(J - 1) & 1], (uint32_t)(((J - 1) >> 1) & 1));
-    __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tbase, 512);
 }
 
