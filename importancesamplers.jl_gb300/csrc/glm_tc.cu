@@ -33,8 +33,12 @@
 // [1, 2], one FMA per pair and one log per 32 (each factor rounds once, like a
 // log would). A log1p per pair, eight epilogue warps and a cold CTA per row
 // tile took 2,384 us at 65,536 samples x 10,000 observations, d = 32 (BF16x3
-// logistic), and 103 us at 50,000 x 500, d = 64 (Gaussian). Every wait is
-// bounded; a timeout sets the sticky error word.
+// logistic), now 315 (426 with the bounds of a ragged tile tested per pair in
+// every tile; 512 row tiles leave the fourth wave of 152 a third full), and 103 us
+// at 50,000 x 500, d = 64 (Gaussian), now 20. Every wait is bounded; a timeout
+// sets the sticky error word.
+#include <type_traits>
+
 #include "issm_device.cuh"
 #include "issm_internal.h"
 #include "tcgen05.cuh"
@@ -316,39 +320,48 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
             for (int c = 0; c < kGlmPartCols; c += 32) {
                 const int o0 = t * kGlmCols + part * kGlmPartCols + c;
                 if (o0 >= p.nobs) break;
-                float v[32], y[32];
-                const bool full = o0 + 32 <= p.nobs;
-                if (full && yvec) {
-#pragma unroll
-                    for (int u = 0; u < 32; u += 4) {
-                        const float4 f = __ldg(reinterpret_cast<const float4 *>(p.y + o0 + u));
-                        y[u] = f.x; y[u + 1] = f.y; y[u + 2] = f.z; y[u + 3] = f.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int u = 0; u < 32; ++u) y[u] = o0 + u < p.nobs ? __ldg(p.y + o0 + u) : 0.f;
-                }
+                float v[32], s[4] = {0.f, 0.f, 0.f, 0.f};
                 tc::tmem_ld32(tbase + ((uint32_t)(32 * qd) << 16) +
                                   (uint32_t)((int)(j & 1) * kGlmCols + part * kGlmPartCols + c), v);
-                float s[4] = {0.f, 0.f, 0.f, 0.f};
-                if (logistic) {
-                    // y eta - max(eta, 0) - log(1 + t); the product of (1 + t) stays below 2^32
+                // FULL: 32 observations, y read 16 bytes at a time; no test per pair
+                auto terms = [&](auto full, auto kind) {
+                    constexpr bool FULL = decltype(full)::value, LOGISTIC = decltype(kind)::value;
                     float q[4] = {1.f, 1.f, 1.f, 1.f};
 #pragma unroll
-                    for (int u = 0; u < 32; ++u) {
-                        const float eta = v[u];
-                        const float tt = full || o0 + u < p.nobs ? exp2_fast(-1.44269504f * fabsf(eta)) : 0.f;
-                        q[u & 3] = fmaf(q[u & 3], tt, q[u & 3]);
-                        const float z = fmaf(y[u], eta, -fmaxf(eta, 0.f));
-                        s[u & 3] += full || o0 + u < p.nobs ? z : 0.f;
-                    }
-                    s[0] -= logf((q[0] * q[1]) * (q[2] * q[3]));
-                } else {
+                    for (int u0 = 0; u0 < 32; u0 += 4) {
+                        float y[4];
+                        if constexpr (FULL) {
+                            const float4 f = __ldg(reinterpret_cast<const float4 *>(p.y + o0 + u0));
+                            y[0] = f.x; y[1] = f.y; y[2] = f.z; y[3] = f.w;
+                        } else {
 #pragma unroll
-                    for (int u = 0; u < 32; ++u) {
-                        const float r = full || o0 + u < p.nobs ? y[u] - v[u] : 0.f;
-                        s[u & 3] = fmaf(r, r, s[u & 3]);
+                            for (int e = 0; e < 4; ++e) y[e] = o0 + u0 + e < p.nobs ? __ldg(p.y + o0 + u0 + e) : 0.f;
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const bool in = FULL || o0 + u0 + e < p.nobs;
+                            const float eta = v[u0 + e];
+                            if constexpr (LOGISTIC) {
+                                // y eta - max(eta, 0) - log(1 + t); the product of (1 + t) stays below 2^32
+                                const float tt = in ? exp2_fast(-1.44269504f * fabsf(eta)) : 0.f;
+                                q[e] = fmaf(q[e], tt, q[e]);
+                                const float z = fmaf(y[e], eta, -fmaxf(eta, 0.f));
+                                s[e] += in ? z : 0.f;
+                            } else {
+                                const float r = in ? y[e] - eta : 0.f;
+                                s[e] = fmaf(r, r, s[e]);
+                            }
+                        }
                     }
+                    if constexpr (LOGISTIC) s[0] -= logf((q[0] * q[1]) * (q[2] * q[3]));
+                };
+                const bool full = o0 + 32 <= p.nobs && yvec;
+                if (logistic) {
+                    if (full) terms(std::true_type(), std::true_type());
+                    else terms(std::false_type(), std::true_type());
+                } else {
+                    if (full) terms(std::true_type(), std::false_type());
+                    else terms(std::false_type(), std::false_type());
                 }
                 acc.add((s[0] + s[1]) + (s[2] + s[3]));
             }
