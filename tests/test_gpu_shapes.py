@@ -402,3 +402,42 @@ def test_round_summary_checks_new_targets(issm, cuda, dtype, size):
     for a, b in zip(*out):
         assert torch.equal(a.nan_to_num(nan=-1.0) if a.is_floating_point() else a,
                            b.nan_to_num(nan=-1.0) if b.is_floating_point() else b)
+
+
+@pytest.mark.parametrize("d", [5, 8, 12, 16, 24, 33, 40, 64])
+@pytest.mark.parametrize("n", [1, 127, 300, 20001])
+def test_row_access_widths(issm, cuda, d, n):
+    """Samples on 4- and 16-byte boundaries (read 4 and 16 bytes at a time) give
+    bitwise the numbers of the aligned array: density of one and of several
+    components, the paired tiles and the moments."""
+    rng = np.random.default_rng(d)
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    x = torch.randn(n, d, device=cuda, generator=gen)
+    lw = torch.randn(n, device=cuda, generator=gen)
+    shift = torch.tensor(0.1 * rng.normal(size=d), device=cuda)
+
+    def offset(k):
+        base = torch.empty(n * d + 8, device=cuda)
+        y = base[k:k + n * d].view(n, d)
+        y.copy_(x)
+        return y
+
+    def numbers(y, prec):
+        out = list(issm.ops.weighted_moments(y, lw, issm.ops.logweight_summary(lw), shift, precision=prec))
+        for k in (1, 3, 21):
+            out.append(issm.ops.mixture_logdensity(banks[k], issm.ops.denominator(
+                issm.native.DENOM_FULL, torch.zeros(k, device=cuda)), y, precision=prec))
+        return [t.clone() for t in out]
+
+    banks = {}
+    for k in (1, 3, 21):
+        props = [issm.FactorGaussian(rng.normal(size=d).astype(np.float32),
+                                     (np.eye(d) + 0.1 * np.tril(rng.normal(size=(d, d)), -1)).astype(np.float32))
+                 for _ in range(k)]
+        banks[k] = issm.pack_proposals(props, cuda)
+        banks[k].attach_inverse_factors()
+    for prec in (issm.native.PREC_BF16, issm.native.PREC_TF32):
+        want = numbers(x, prec)
+        for off in (1, 4):
+            for a, b in zip(want, numbers(offset(off), prec)):
+                assert torch.equal(a, b)
