@@ -15,7 +15,10 @@ __device__ __forceinline__ int row_access(const float *x, int d) {
 // Coordinates c .. c + 7 (c a multiple of 8) of sample i into registers, zeros
 // beyond d and for an inactive sample. One 32-byte request per lane: two 16-byte
 // ones each ask for half of a lane's sector, and 256 MB read that way came at 4.35
-// TB/s against 6.3 for requests of whole sectors.
+// TB/s against 6.3 for requests of whole sectors. The samples leave L2 first: a run's
+// retained rows (512 MB at 2M x 64) pass through it twice a round, and kept out what
+// every round rereads, instructions included: 11.06 -> 10.53 ms of device time a run,
+// the fit between the passes 47 -> 43 us, an operand preparation 9.9 -> 6.5.
 __device__ __forceinline__ void load_group(float (&v)[8], const float *__restrict__ x, int64_t i, bool active, int d,
                                            int c, int access) {
     const float *src = x + i * d + c;
@@ -23,7 +26,7 @@ __device__ __forceinline__ void load_group(float (&v)[8], const float *__restric
     for (int m = 0; m < 8; ++m) v[m] = 0.f;
     if (access == 32) {
         if (active && c < d)
-            asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            asm volatile("ld.global.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                          : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]),
                            "=f"(v[7])
                          : "l"(src));
