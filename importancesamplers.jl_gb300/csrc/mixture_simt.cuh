@@ -676,6 +676,12 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
         stage_request<T, D, FACTOR>(comps + (size_t)buf * p.chunk * Ly::kStride, p, p.first_slot + k0,
                                     min(p.chunk, nslots - k0));
     };
+    // a draw's component: staged if it is one of the denominator's terms (a prefix
+    // may stop before a drawn slot, and a plain draw stages none), else null
+    auto staged = [&](int slot) -> const T * {
+        const int at = slot - p.first_slot;
+        return p.resident && at >= 0 && at < nslots ? comps + (size_t)at * Ly::kStride : nullptr;
+    };
     const bool drawn = p.mode == kModeRound || p.mode == kModeDraw;
     const T *rows_in = drawn ? p.normals : p.x;
     auto tile_row = [&](int it) -> int64_t { return ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * TR; };
@@ -734,7 +740,7 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                 const int64_t i = row0 + si + s * GT;
                 load_row<T, D>(rows_in + (size_t)(ok[s] ? i : 0) * d, d, vec, x[s]);
                 if (drawn && ok[s]) {
-                    const T *c = p.resident && nslots > 0 ? comps + (size_t)gen[s] * Ly::kStride : nullptr;
+                    const T *c = staged(gen[s]);
                     ok[s] = draw_registers<T, D>(p, gen[s], c, draw_multiplier(p, i, gen[s], grp == 0), x[s]);
                     if (grp == 0) {
                         if (!ok[s])
@@ -751,7 +757,7 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                 for (int s = 0; s < S; ++s)
                     if (ok[s]) {
                         const int64_t i = row0 + si + s * GT;
-                        const T *c = p.resident && nslots > 0 ? comps + (size_t)gen[s] * Ly::kStride : nullptr;
+                        const T *c = staged(gen[s]);
                         T *row = tile + (size_t)(si + s * GT) * LX;
                         if (!draw_row<T, D, FACTOR>(p, gen[s], c, draw_multiplier(p, i, gen[s]), 0, 1, row, row)) {
                             record_failure(p.failures, p.index_base + i + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
@@ -765,7 +771,7 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                 if (grp == 0) s_bad[si] = 0;
                 __syncthreads();
                 if (ok[0]) {
-                    const T *c = p.resident ? comps + (size_t)gen[0] * Ly::kStride : nullptr;
+                    const T *c = staged(gen[0]);
                     if (!draw_row<T, D, FACTOR>(p, gen[0], c, mult[si], grp, KS, tile + (size_t)si * LX,
                                                 drawn_tile + (size_t)si * LX))
                         s_bad[si] = 1;

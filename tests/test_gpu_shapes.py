@@ -441,3 +441,38 @@ def test_row_access_widths(issm, cuda, d, n):
         for off in (1, 4):
             for a, b in zip(want, numbers(offset(off), prec)):
                 assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k,terms,dof", [(100, 3, 8, 3, None), (5000, 16, 8, 3, 5.0), (1000, 12, 40, 1, None),
+                                             (700, 24, 8, 3, None), (333, 33, 60, 2, 4.0), (200_003, 7, 9, 4, None),
+                                             (257, 64, 70, 65, None)])
+def test_prefix_round_draws_every_slot(issm, orc, cuda, dtype, n, d, k, terms, dof):
+    """A round over a prefix of the bank whose samples come from every slot: the
+    draws of slots beyond the prefix equal the separate draw's, the weights the
+    separate prefix density's, bitwise, and the oracle's (tolerances as
+    test_simt_density_shapes)."""
+    rng = np.random.default_rng(n + terms)
+    db, ob = _factor_bank(issm, orc, rng, d, k, dtype, cuda, dof)
+    tdt = torch.float32 if dtype == np.float32 else torch.float64
+    slots = rng.integers(0, k, size=n).astype(np.int32)
+    slots[:k] = np.arange(k)
+    ts = torch.tensor(slots, device=cuda)
+    normals = torch.tensor(rng.normal(size=n * d).astype(dtype), device=cuda)
+    rad = {}
+    if dof:
+        rad = dict(radial_normals=torch.tensor(rng.normal(size=n * 8).astype(dtype), device=cuda), rn_stride=8,
+                   radial_uniforms=torch.tensor(rng.random(size=n * 8).astype(dtype), device=cuda), ru_stride=8)
+    coef = np.log(rng.dirichlet(np.ones(k))).astype(dtype)
+    tc = torch.tensor(coef, device=cuda)
+    den = issm.ops.denominator(issm.native.DENOM_PREFIX, tc, terms=terms)
+    db.proposal_ids = torch.arange(1, k + 1, device=cuda)
+    fail = issm.ops.new_failures(cuda)
+    x, lw, pid = issm.ops.mis_round(db, den, ts, normals, failures=fail, **rad)
+    assert torch.equal(x, issm.ops.draw(db, normals, n, slots=ts, **rad))
+    assert torch.equal(lw, -issm.ops.mixture_logdensity(db, den, x, slots=ts))
+    assert torch.equal(pid, ts.long() + 1) and int(fail[0].item()) == 0
+    exp, _, _ = orc.mixture_logdensity(ob, x.double().cpu().numpy().reshape(-1), orc.DENOM_PREFIX,
+                                       coef.astype(np.float64), terms=terms, slots=slots)
+    tol = 1e-12 if dtype == np.float64 else 2e-5
+    assert np.all(np.abs(lw.double().cpu().numpy() + exp) <= tol * np.maximum(1.0, np.abs(exp)))
