@@ -306,6 +306,9 @@ __global__ void __launch_bounds__(kQThreads) quantile_setup_kernel(const T *__re
 // ---- choosing a bin ------------------------------------------------------------
 // The first bin whose cumulative weight (from `below`) exceeds thr; every
 // thread returns it (kQBins: none) with the weight below it and its count.
+// A thread's starting sum is associated differently from the sum that the thread
+// before it ends with, so it may exceed thr by a rounding though no earlier bin
+// did: the weight below the bin is then thr itself, as everywhere a sum is chosen.
 __device__ __forceinline__ int q_choose(const QBins *bins, double below, double thr, double *under, unsigned *count) {
     __shared__ int s_bin;
     __shared__ double s_under;
@@ -324,7 +327,7 @@ __device__ __forceinline__ int q_choose(const QBins *bins, double below, double 
     for (int k = 0; k < kQPer; ++k) {
         if (hit == kQBins && v[k] > 0.0 && cum + v[k] > thr) {
             hit = threadIdx.x * kQPer + k;
-            at = cum;
+            at = fmin(cum, thr);
         }
         cum += v[k];
     }
@@ -575,11 +578,14 @@ __global__ void __launch_bounds__(kQThreads) quantile_gather_kernel(const T *__r
     }
 }
 
-// lower + f (upper - lower) as _weighted_quantile forms it (src/statistics.jl:140-153)
-__device__ __forceinline__ double q_interpolate(double lo, double up, double f) {
+// lower + f (upper - lower) as _weighted_quantile forms it (src/statistics.jl:140-153),
+// f = (thr - at) / w with at <= thr < at + w up to the rounding of the sums
+__device__ __forceinline__ double q_interpolate(double lo, double up, double thr, double at, double w) {
+    const double f = fmin((thr - at) / w, 1.0);
     if (f == 0.0) return lo;
+    if (f == 1.0) return up;
     const double diff = up - lo;
-    return isfinite(diff) ? lo + f * diff : (1.0 - f) * lo + f * up;
+    return isfinite(diff) ? fmin(lo + f * diff, up) : (1.0 - f) * lo + f * up;
 }
 
 // ---- one CTA per problem: sort the interval's samples, select, interpolate --------------
@@ -602,7 +608,7 @@ __global__ void __launch_bounds__(kQThreads) quantile_finish_kernel(int d, const
             const double up = (double)QK::value(s.ka);
             const double w = qweight((double)lw[s.first], summary[0], 1.0 / summary[1]);
             double v = up;
-            if (klow != 0ull && s.below + w > s.thr) v = q_interpolate((double)QK::value(klow), up, (s.thr - s.below) / w);
+            if (klow != 0ull && s.below + w > s.thr) v = q_interpolate((double)QK::value(klow), up, s.thr, s.below, w);
             out[pr] = (double)(T)v;
         }
         return;
@@ -654,7 +660,7 @@ __global__ void __launch_bounds__(kQThreads) quantile_finish_kernel(int d, const
         const double we = w[ord[e]];
         if (hit == m && cum + we > s.thr) {
             hit = e;
-            at = cum;
+            at = fmin(cum, s.thr);  // as in q_choose
         }
         cum += we;
     }
@@ -666,7 +672,7 @@ __global__ void __launch_bounds__(kQThreads) quantile_finish_kernel(int d, const
         double v = up;
         if (hit > 0 || klow != 0ull) {
             const double lo = (double)QK::value(hit > 0 ? key[ord[hit - 1]] : klow);
-            v = q_interpolate(lo, up, (s.thr - at) / w[ord[hit]]);
+            v = q_interpolate(lo, up, s.thr, at, w[ord[hit]]);
         }
         out[pr] = (double)(T)v;
     } else if (tid == 0) {  // the sorted sums rounded below the bins': the interval's last sample

@@ -476,3 +476,44 @@ def test_prefix_round_draws_every_slot(issm, orc, cuda, dtype, n, d, k, terms, d
                                        coef.astype(np.float64), terms=terms, slots=slots)
     tol = 1e-12 if dtype == np.float64 else 2e-5
     assert np.all(np.abs(lw.double().cpu().numpy() + exp) <= tol * np.maximum(1.0, np.abs(exp)))
+
+
+# The cumulative weights are sums of at most n positive FP64 terms of total one, in
+# any order: (n + 8) eps covers them, the weights' own roundings and the threshold's.
+# Within that much weight of the exact threshold lie the only samples that a
+# quantile may be formed from, and an interpolation stays between two neighbours.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("kind", ["narrow", "tiny_top", "tiny_both", "ties"])
+@pytest.mark.parametrize("n", [300, 4000, 30_000])
+def test_weighted_quantile_between_neighbours(issm, cuda, dtype, kind, n):
+    """Weights that span more than forty in the logarithm, the largest or the
+    smallest values next to weightless: every quantile lies between the samples
+    that hold its threshold."""
+    rng = np.random.default_rng(n)
+    probs = [0.0, 1e-12, 0.05, 0.5, 0.95, 1.0 - 1e-12, 1.0]
+    eps = 2.0**-52
+    for rep in range(4):
+        x = 3.0 * rng.normal(size=n)
+        if kind == "ties":
+            x = np.round(2.0 * x) / 2.0
+        lw = -1.5 * x * x
+        if kind in ("tiny_top", "tiny_both"):
+            small = (x > np.quantile(x, 0.9)) | ((x < np.quantile(x, 0.1)) & (kind == "tiny_both"))
+            lw = np.where(small, -45.0 - 10.0 * rng.random(n), rng.normal(size=n))
+        d = 24  # affine images: other bins for the same order or its reverse
+        X = x[:, None] * rng.uniform(0.3, 3.0, size=d) * rng.choice([-1.0, 1.0], size=d) + 5.0 * rng.normal(size=d)
+        tx, tl = torch.tensor(X, device=cuda).to(dtype), torch.tensor(lw, device=cuda).to(dtype)
+        got = issm.quantile(issm.WeightedSamples(tx, tl), probs).cpu().numpy()
+        l64 = tl.double().cpu().numpy()
+        w = np.exp((l64 - l64.max()).astype(np.longdouble))
+        w /= w.sum()
+        V = tx.double().cpu().numpy()
+        delta = (n + 8) * eps
+        for c in range(d):
+            at = np.argsort(V[:, c], kind="stable")
+            v, cum = V[at, c], np.cumsum(w[at])
+            for j, p in enumerate(probs):
+                thr = np.longdouble(p) * (cum[-1] - w[at[0]]) + w[at[0]]
+                lo = max(int(np.searchsorted(cum, thr - delta, side="right")) - 1, 0)
+                hi = min(int(np.searchsorted(cum, thr + delta, side="right")), n - 1)
+                assert v[lo] <= got[j, c] <= v[hi], (kind, n, rep, c, p, v[lo], got[j, c], v[hi])
