@@ -28,15 +28,15 @@
 //     all of them fit, else stream through a ring of bulk copies;
 //   * warps 5-20, four per TMEM lane quadrant and 64 columns each, reduce the
 //     other accumulator.
-// The epilogue bounds it, so a pair costs one MUFU and five FP32 operations:
-// with t = e^-|eta|, sum log(1 + t) is the logarithm of a product of factors in
-// [1, 2], one FMA per pair and one log per 32 (each factor rounds once, like a
-// log would). A log1p per pair, eight epilogue warps and a cold CTA per row
-// tile took 2,384 us at 65,536 samples x 10,000 observations, d = 32 (BF16x3
-// logistic), now 315 (426 with the bounds of a ragged tile tested per pair in
-// every tile; 512 row tiles leave the fourth wave of 152 a third full), and 103 us
-// at 50,000 x 500, d = 64 (Gaussian), now 20. Every wait is bounded; a timeout
-// sets the sticky error word.
+// The epilogue bounds it, so a pair costs one MUFU and eight FP32 operations: with
+// t = e^-|eta|, sum log(1 + t) is log1p of a product of factors 1 + t, carried less
+// one, P <- P + t + P t, so that a small t keeps its relative accuracy (the factors
+// themselves would round it at 2^-24 of one: at |eta| = 17 all of it), and one log1p
+// per 32. A log1p per pair, eight epilogue warps and a cold CTA per row tile took
+// 2,384 us at 65,536 samples x 10,000 observations, d = 32 (BF16x3 logistic), now 367
+// (512 row tiles leave the fourth wave of 152 a third full), and 103 us at 50,000 x
+// 500, d = 64 (Gaussian), now 20. Every wait is bounded; a timeout sets the sticky
+// error word.
 #include <type_traits>
 
 #include "issm_device.cuh"
@@ -126,11 +126,21 @@ struct GlmPair {
     __device__ __forceinline__ double value() const { return isfinite(h) ? (double)h + (double)l : (double)h; }
 };
 
-__device__ __forceinline__ float exp2_fast(float v) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
+// e^-|v| with the rounding of |v| log2(e) put back: 2^p of the product p rounded
+// down, times 1 + r with r = -|v| - p ln 2 >= 0 (log2(e) is rounded up for that), so a
+// small term keeps its relative accuracy. Saturation makes r 0 for infinite v. The
+// largest error is 3.3 units of 2^-24 for |v| up to 30 (5.5 up to 85); without the
+// correction 16 at 17 and 63 at 85. expf (2.6) makes the call a quarter slower,
+// and the log target's error is the same.
+__device__ __forceinline__ float exp_neg(float v) {
+    const float a = -fabsf(v), p = __fmul_rd(a, 0x1.715478p+0f);
+    float t;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(p));
+    const float r = __saturatef(fmaf(p, -0x1.62e43p-1f, a));
+    return fmaf(t, r, t);
 }
+// (1 + p)(1 + t) - 1
+__device__ __forceinline__ float join_log1p(float p, float t) { return fmaf(p, t, p + t); }
 
 template <int KIND, int SPLIT, int DP>
 __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
@@ -326,7 +336,7 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
                 // FULL: 32 observations, y read 16 bytes at a time; no test per pair
                 auto terms = [&](auto full, auto kind) {
                     constexpr bool FULL = decltype(full)::value, LOGISTIC = decltype(kind)::value;
-                    float q[4] = {1.f, 1.f, 1.f, 1.f};
+                    float q[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                     for (int u0 = 0; u0 < 32; u0 += 4) {
                         float y[4];
@@ -342,9 +352,9 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
                             const bool in = FULL || o0 + u0 + e < p.nobs;
                             const float eta = v[u0 + e];
                             if constexpr (LOGISTIC) {
-                                // y eta - max(eta, 0) - log(1 + t); the product of (1 + t) stays below 2^32
-                                const float tt = in ? exp2_fast(-1.44269504f * fabsf(eta)) : 0.f;
-                                q[e] = fmaf(q[e], tt, q[e]);
+                                // y eta - max(eta, 0) - log(1 + t); q, the product of (1 + t)
+                                // less one, stays below 2^32
+                                q[e] = join_log1p(q[e], in ? exp_neg(eta) : 0.f);
                                 const float z = fmaf(y[e], eta, -fmaxf(eta, 0.f));
                                 s[e] += in ? z : 0.f;
                             } else {
@@ -353,7 +363,7 @@ __global__ void __launch_bounds__(kGlmThreads, 1) glm_tc_kernel(GlmParams p) {
                             }
                         }
                     }
-                    if constexpr (LOGISTIC) s[0] -= logf((q[0] * q[1]) * (q[2] * q[3]));
+                    if constexpr (LOGISTIC) s[0] -= log1pf(join_log1p(join_log1p(q[0], q[1]), join_log1p(q[2], q[3])));
                 };
                 const bool full = o0 + 32 <= p.nobs && yvec;
                 if (logistic) {

@@ -517,3 +517,43 @@ def test_weighted_quantile_between_neighbours(issm, cuda, dtype, kind, n):
                 lo = max(int(np.searchsorted(cum, thr - delta, side="right")) - 1, 0)
                 hi = min(int(np.searchsorted(cum, thr + delta, side="right")), n - 1)
                 assert v[lo] <= got[j, c] <= v[hi], (kind, n, rep, c, p, v[lo], got[j, c], v[hi])
+
+
+# log(1 + e^-|eta|) of well-separated observations, each a small positive term. With
+# u = 2^-24 an exponential is within 4 u, the joined factors of 32 observations within
+# 2 u per step (ten steps) and their logarithm within 2 u: 32 u of the sum of the
+# terms. The rest of the log target is exact (predictors are products of bf16 numbers,
+# y eta - max(eta, 0) is zero) but for the final rounding, 2 u of the value.
+@pytest.mark.parametrize("form", ["bf16", "tf32", "bf16x1"])
+@pytest.mark.parametrize("case", ["8", "12", "14", "17", "mixed", "rare"])
+@pytest.mark.parametrize("nobs", [31, 10_000])
+def test_glm_well_separated_observations(issm, cuda, form, case, nobs):
+    rng = np.random.default_rng(nobs)
+    if case == "mixed":
+        mag = rng.integers(8 * 8, 25 * 8, size=nobs) / 8.0
+    elif case == "rare":
+        mag = rng.integers(6 * 8, 14 * 8, size=nobs) / 8.0
+    else:
+        mag = np.full(nobs, float(case))
+    sign = np.ones(nobs) if case in ("8", "17") else -np.ones(nobs) if case == "rare" else rng.choice([-1.0, 1.0], size=nobs)
+    X = np.stack([mag * sign, np.zeros(nobs)], axis=1)
+    y = (sign > 0).astype(np.float64)
+    B = np.array([[1.0, 0.0], [0.5, 0.0], [1.0, 2.0]] * 50, dtype=np.float32)
+    prec = {"bf16": issm.native.PREC_BF16, "tf32": issm.native.PREC_TF32, "bf16x1": issm.native.PREC_BF16X1}[form]
+    bound = issm.LogisticRegressionTarget(X, y, 10.0).bind(cuda, torch.float32)
+    got = bound.evaluate(torch.tensor(B, device=cuda), precision=prec).double().cpu().numpy()
+    tail = np.log1p(np.exp(-np.abs(B.astype(np.float64)[:, :1] * X[:, 0]))).sum(1)
+    want = -tail - np.log(2 * np.pi * 10.0) - (B.astype(np.float64) ** 2).sum(1) / 20.0
+    u = 2.0**-24
+    assert np.all(np.abs(got - want) <= 32 * u * tail + 2 * u * np.abs(want))
+
+
+def test_glm_infinite_predictors(issm, cuda):
+    """Predictors that overflow: -inf where every observation disagrees with an
+    infinite predictor's side, NaN only where the likelihood is undefined."""
+    X = np.array([[3.0e38, 0.0], [3.0e38, 0.0]])
+    B = torch.tensor([[4.0, 0.0], [-4.0, 0.0], [float("nan"), 0.0]], device=cuda)
+    for prec in (issm.native.PREC_TF32, issm.native.PREC_BF16X1):
+        bound = issm.LogisticRegressionTarget(X, np.ones(2), 10.0).bind(cuda, torch.float32)
+        got = bound.evaluate(B, precision=prec).cpu().numpy()
+        assert np.isnan(got[0]) and got[1] == -np.inf and np.isnan(got[2])
