@@ -58,8 +58,9 @@ __global__ void target_simple_kernel(issm_target t, const T *__restrict__ x, int
 // linear predictors of RS samples x 4 observations while the coordinates pass
 // through shared memory (X is nobs x d column-major, so a coordinate's
 // observations are contiguous). The logistic terms use
-// y eta - max(eta, 0) - log(1 + e^-|eta|) with the factors (1 + e^-|eta|),
-// each in [1, 2], multiplied into a product whose log is taken once per 64.
+// y eta - max(eta, 0) - log(1 + t), t = e^-|eta|, with the factors (1 + t)
+// multiplied into a product, carried less one (P <- P + t + P t) so that small
+// terms keep their relative accuracy, whose log1p is taken once per 64.
 // Sums of FP32 terms are carried as unevaluated pairs.
 //
 // Bound by FMA issue with shared operands (FP32) or the FP64 pipe. A warp per
@@ -67,7 +68,7 @@ __global__ void target_simple_kernel(issm_target t, const T *__restrict__ x, int
 // observations, d = 33, FP32.
 constexpr int kRegObs = 64;   // observations per step
 constexpr int kRegDim = 64;   // coordinates staged at a time
-constexpr int kRegFlush = 16; // steps between logs of the product (4 factors each)
+constexpr int kRegFlush = 16; // steps between log1ps of the product (4 factors each)
 
 template <typename T> struct RegSum {  // FP64: plain
     T h = T(0);
@@ -117,11 +118,11 @@ __global__ void __launch_bounds__(256) target_regression_kernel(issm_target t, c
     const int64_t s0 = (int64_t)blockIdx.x * TS;
     const int rows = (int)min((int64_t)TS, n - s0);
     RegSum<T> acc[RS];
-    T prod[RS];
+    T prod[RS];  // less one
     T bb[RS];
 #pragma unroll
     for (int i = 0; i < RS; ++i) {
-        prod[i] = T(1);
+        prod[i] = T(0);
         bb[i] = T(0);
     }
     int steps = 0;
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(256) target_regression_kernel(issm_target t, c
                 const T e = eta[i][j];
                 if (logistic) {
                     const T f = dexp(-fabs(e));
-                    prod[i] += prod[i] * f;
+                    prod[i] += prod[i] * f + f;
                     sum += yv[j] * e - (e > T(0) ? e : isnan(e) ? e : T(0));
                 } else {
                     const T r = yv[j] - e;
@@ -186,8 +187,8 @@ __global__ void __launch_bounds__(256) target_regression_kernel(issm_target t, c
         if (logistic && (++steps % kRegFlush == 0 || o0 + kRegObs >= nobs))
 #pragma unroll
             for (int i = 0; i < RS; ++i) {
-                acc[i].add(-dlog(prod[i]));
-                prod[i] = T(1);
+                acc[i].add(-dlog1p(prod[i]));
+                prod[i] = T(0);
             }
     }
 #pragma unroll

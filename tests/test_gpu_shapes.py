@@ -557,3 +557,35 @@ def test_glm_infinite_predictors(issm, cuda):
         bound = issm.LogisticRegressionTarget(X, np.ones(2), 10.0).bind(cuda, torch.float32)
         got = bound.evaluate(B, precision=prec).cpu().numpy()
         assert np.isnan(got[0]) and got[1] == -np.inf and np.isnan(got[2])
+
+
+# The SIMT form of the same, in both types: exponentials within 4 u, 64 factors per
+# logarithm at 2 u each, the logarithm 2 u, the sums of logarithms error-free (FP32) or one
+# rounding per 64 observations and five of the lanes' (FP64): (140 + nobs / 1024) u of
+# the sum of the terms; the constant, the prior and the total in the type: 4 u of their sizes.
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("case", ["8", "12", "17", "25", "mixed", "rare"])
+@pytest.mark.parametrize("nobs,n", [(31, 40), (10_000, 40), (3000, 5000)])
+def test_simt_well_separated_observations(issm, cuda, dtype, case, nobs, n):
+    rng = np.random.default_rng(nobs + n)
+    if case == "mixed":
+        mag = rng.integers(8 * 8, 25 * 8, size=nobs) / 8.0
+    elif case == "rare":
+        mag = rng.integers(6 * 8, 14 * 8, size=nobs) / 8.0
+    else:
+        mag = np.full(nobs, float(case))
+    sign = -np.ones(nobs) if case in ("8", "17", "rare") else rng.choice([-1.0, 1.0], size=nobs)
+    X = np.stack([mag * sign, np.zeros(nobs)], axis=1)
+    B = np.zeros((n, 2), dtype=dtype)
+    B[:, 0] = np.where(np.arange(n) % 2, 1.0, 0.5)
+    B[:, 1] = np.arange(n) % 3
+    tdt = torch.float32 if dtype == np.float32 else torch.float64
+    bound = issm.LogisticRegressionTarget(X, (sign > 0).astype(np.float64), 10.0).bind(cuda, tdt)
+    got = bound.evaluate(torch.tensor(B, device=cuda)).cpu().numpy().astype(np.longdouble)
+    B = B.astype(np.longdouble)
+    slope, row = np.unique(B[:, 0], return_inverse=True)
+    tail = np.log1p(np.exp(-np.abs(slope[:, None] * X[:, 0]))).sum(1)[row]
+    const, prior = -np.log(2 * np.longdouble(np.pi) * 10), -(B ** 2).sum(1) / 20
+    u = float(np.finfo(dtype).eps) / 2
+    bound = (140 + nobs / 1024) * u * tail + 4 * u * (tail + abs(const) + np.abs(prior))
+    assert np.all(np.abs(got - (const + prior - tail)) <= bound)
