@@ -279,7 +279,7 @@ __device__ const LogEntry kLogTable[128] = {
     {0x1.0080400000000p-1, 0x1.61e3f01a46800p-1, -0x1.cc9436e4fb135p-44},
 };
 
-// e^x for -37.5 < x <= 0: x = k ln 2 / 128 + r, |r| <= ln 2 / 256, e^r - 1 to degree 5
+// e^x for -60 < x <= 0: x = k ln 2 / 128 + r, |r| <= ln 2 / 256, e^r - 1 to degree 5
 __device__ __forceinline__ double table_exp(double x) {
     const double t = fma(x, 0x1.71547652b82fep+7, 0x1.8p52);  // 128 / ln 2: k in the low mantissa bits
     const int k = __double2loint(t);

@@ -74,8 +74,9 @@ template <> __device__ __forceinline__ double qnan<double>() { return __longlong
 // Online log-sum-exp over terms: one exp per term, exact special values
 // (NaN propagates, -Inf terms vanish, equal infinities collapse as logaddexp).
 // FP64 exponentials are dear on this GPU: a term too small to change the sum
-// takes none. s >= 1 once a term is in, so e^-37.5 < 2^-54 rounds away when
-// added to it, and s e^-60 when added to 1 (s counts at most the terms).
+// takes none. s >= 1 once a term is in, so a term of e^-37.5 < 2^-54 rounds away
+// when added to it; a sum that a new maximum scales down may hold a count of terms,
+// so it is dropped from e^-60 on only (10^10 terms below half an ulp of 1).
 template <typename T> struct LseState {
     T m = -num<T>::inf();
     T s = T(0);
@@ -91,8 +92,8 @@ template <typename T> struct LseState {
                 const bool up = t > m;
                 const T gap = up ? m - t : t - m;  // <= 0; NaN for equal infinities
                 const uint32_t g = (uint32_t)__double2hiint(gap) & 0x7fffffffu;
-                // beyond 37.5 a term is below half an ulp of the sum; equal infinities count as equal
-                T e = g < 0x4042c000u ? table_exp(gap) : t == m ? T(1) : T(0);
+                // 37.5 and 60 by their leading words; equal infinities count as equal
+                T e = g < (up ? 0x404e0000u : 0x4042c000u) ? table_exp(gap) : t == m ? T(1) : T(0);
                 s = fma(up ? s : e, up ? e : T(1), up ? T(1) : s);
                 m = up ? t : m;
             }

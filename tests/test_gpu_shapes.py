@@ -589,3 +589,24 @@ def test_simt_well_separated_observations(issm, cuda, dtype, case, nobs, n):
     u = float(np.finfo(dtype).eps) / 2
     bound = (140 + nobs / 1024) * u * tail + 4 * u * (tail + abs(const) + np.abs(prior))
     assert np.all(np.abs(got - (const + prior - tail)) <= bound)
+
+
+# The smaller terms' sum is a whole number of e^-gap, exact; the exponential, the last
+# sum and the logarithm round as in test_f64_log_sum_exp, without its count of terms.
+@pytest.mark.parametrize("k", [1025, 4001])
+@pytest.mark.parametrize("gap", [37.4, 37.6, 45.0, 59.9, 60.1])
+@pytest.mark.parametrize("last", [True, False])
+def test_f64_log_sum_exp_of_many_small_terms(issm, cuda, k, gap, last):
+    """Many equal terms and one that is `gap` above them, after them or before."""
+    db = issm.pack_proposals([issm.FactorGaussian(np.zeros(2), np.eye(2))] * k, cuda)
+    x = np.linspace(0.0, 0.5, 20).reshape(10, 2)
+    coef = np.full(k, -gap)
+    coef[-1 if last else 0] = 0.0
+    den = issm.ops.denominator(issm.native.DENOM_FULL, torch.tensor(coef, device=cuda))
+    got = issm.ops.mixture_logdensity(db, den, torch.tensor(x, device=cuda)).cpu().numpy()
+    xl = x.astype(np.longdouble)
+    lq = -np.log(2 * np.longdouble(np.pi)) - 0.5 * (xl * xl).sum(1)
+    want = (lq + np.log1p((k - 1) * np.exp(-np.longdouble(gap)))).astype(np.float64)
+    # after the maximum each small term meets a sum of at least 1 and may round away: half an ulp of it each
+    order = 0.0 if last else 2.0**-53 * k
+    assert np.all(np.abs(got - want) <= 2.0**-52 * (16 + 8 * np.abs(lq.astype(np.float64))) + order)
