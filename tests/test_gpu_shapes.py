@@ -610,3 +610,38 @@ def test_f64_log_sum_exp_of_many_small_terms(issm, cuda, k, gap, last):
     # after the maximum each small term meets a sum of at least 1 and may round away: half an ulp of it each
     order = 0.0 if last else 2.0**-53 * k
     assert np.all(np.abs(got - want) <= 2.0**-52 * (16 + 8 * np.abs(lq.astype(np.float64))) + order)
+
+
+# A forward pass over 8-row blocks: the products L_ik W_kj are sums of at most d / 4 + 8
+# rounded terms per thread and two sums across threads, the diagonal block's inverse is
+# a substitution of 8 rows: |L W - I| <= (d / 4 + 26) 2^-24 D |L| |W|, D the block diagonal of
+# |L_ii| |W_ii|, whatever the condition of the rest.
+@pytest.mark.parametrize("d,split", [(16, 8), (24, 16), (40, 16), (48, 32), (63, 16), (64, 16), (64, 32), (64, 40)])
+def test_inverse_factor_residual(issm, cuda, d, split):
+    """Factors whose lower right part is badly conditioned while its part of the
+    inverse stays of order one."""
+    rng = np.random.default_rng(d + split)
+    L = np.eye(d) + np.tril(0.1 * rng.normal(size=(d, d)), -1)
+    low = np.eye(d - split) - np.tril(rng.uniform(0.3, 0.7, size=(d - split, d - split)), -1)
+    L[split:, split:] = low
+    L[split:, :split] = low @ rng.uniform(-1.0, 1.0, size=(d - split, split)) @ L[:split, :split]
+    L = L.astype(np.float32)
+    db = issm.pack_proposals([issm.FactorGaussian(np.zeros(d, dtype=np.float32), L)], cuda)
+    db.attach_inverse_factors()
+    dp = 16 if d <= 16 else 32 if d <= 32 else 64
+    loc, fac = torch.empty(d, device=cuda), torch.empty(d, d, device=cuda)
+    ln, inv = torch.empty(1, device=cuda), torch.empty(dp, dp, device=cuda)
+    L64, fail = L.astype(np.float64), issm.ops.new_failures(cuda)
+    issm.ops.fit_factor(torch.zeros(d, device=cuda, dtype=torch.float64), torch.tensor(L64 @ L64.T, device=cuda),
+                        torch.eye(d, device=cuda), loc, fac, ln, failures=fail, regularization=0.0, out_inverse=inv)
+    pairs = [(L64, db.inverse_factors)]
+    if int(fail[0].item()) == 0:  # else L L^T is not positive definite in FP64 and the fit refused it
+        pairs.append((fac.double().cpu().numpy().T, inv))
+    for factor, inverse in pairs:
+        W = inverse.double().cpu().numpy().reshape(dp, dp)[:d, :d]
+        D = np.zeros((d, d))
+        for b in range(0, d, 8):
+            at = slice(b, min(b + 8, d))
+            D[at, at] = np.abs(factor[at, at]) @ np.abs(W[at, at])
+        bound = (d / 4 + 26) * 2.0**-24 * (D @ (np.abs(factor) @ np.abs(W)))
+        assert np.all(np.abs(factor @ W - np.eye(d)) <= bound)
