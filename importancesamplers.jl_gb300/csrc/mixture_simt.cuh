@@ -676,12 +676,10 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
         stage_request<T, D, FACTOR>(comps + (size_t)buf * p.chunk * Ly::kStride, p, p.first_slot + k0,
                                     min(p.chunk, nslots - k0));
     };
-    // a draw's component: staged if it is one of the denominator's terms (a prefix
-    // may stop before a drawn slot, and a plain draw stages none), else null
-    auto staged = [&](int slot) -> const T * {
-        const int at = slot - p.first_slot;
-        return p.resident && at >= 0 && at < nslots ? comps + (size_t)at * Ly::kStride : nullptr;
-    };
+    // a draw's component: staged where the whole bank is, else null (a prefix may stop
+    // before a drawn slot, a plain draw stages none)
+    const bool whole = p.resident && nslots == p.k;
+    auto staged = [&](int slot) -> const T * { return whole ? comps + (size_t)slot * Ly::kStride : nullptr; };
     const bool drawn = p.mode == kModeRound || p.mode == kModeDraw;
     const T *rows_in = drawn ? p.normals : p.x;
     auto tile_row = [&](int it) -> int64_t { return ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * TR; };
