@@ -733,19 +733,23 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
         T *xs = tile;
         T x[S][XREG ? D : 1];
         if constexpr (DIRECT) {
+            auto put = [&](int s) {
+                const int64_t i = row0 + si + s * GT;
+                if (i >= p.n) return;
+                if (!ok[s]) record_failure(p.failures, p.index_base + i + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
+                if (p.samples_out) store_row<T, D>(p.samples_out + (size_t)i * d, d, vec, x[s]);
+            };
 #pragma unroll
             for (int s = 0; s < S; ++s) {
                 const int64_t i = row0 + si + s * GT;
                 load_row<T, D>(rows_in + (size_t)(ok[s] ? i : 0) * d, d, vec, x[s]);
-                if (drawn && ok[s]) {
-                    const T *c = staged(gen[s]);
-                    ok[s] = draw_registers<T, D>(p, gen[s], c, draw_multiplier(p, i, gen[s], grp == 0), x[s]);
-                    if (grp == 0) {
-                        if (!ok[s])
-                            record_failure(p.failures, p.index_base + i + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
-                        if (p.samples_out) store_row<T, D>(p.samples_out + (size_t)i * d, d, vec, x[s]);
-                    }
-                }
+                if (drawn && ok[s])
+                    ok[s] = draw_registers<T, D>(p, gen[s], staged(gen[s]), draw_multiplier(p, i, gen[s], grp == 0), x[s]);
+                if (drawn && KS == 1) put(s);
+            }
+            if (S == 1 && drawn && KS > 1) {
+                __syncthreads();  // every group has its normals: the samples may take their place
+                if (grp == 0) put(0);
             }
             if (p.mode == kModeDraw) continue;
             if (drawn && KS > 1) __syncthreads();  // the slow path reads the stored samples

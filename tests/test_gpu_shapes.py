@@ -645,3 +645,30 @@ def test_inverse_factor_residual(issm, cuda, d, split):
             D[at, at] = np.abs(factor[at, at]) @ np.abs(W[at, at])
         bound = (d / 4 + 26) * 2.0**-24 * (D @ (np.abs(factor) @ np.abs(W)))
         assert np.all(np.abs(factor @ W - np.eye(d)) <= bound)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k,dof", [(100, 3, 8, None), (5000, 16, 8, 5.0), (20_000, 12, 40, None), (700, 24, 8, None),
+                                       (333, 33, 20, 4.0), (400_003, 7, 3, None)])
+def test_round_in_place(issm, orc, cuda, dtype, n, d, k, dof):
+    """Samples written over the normals they are drawn from: the numbers of
+    separate arrays."""
+    rng = np.random.default_rng(n)
+    db, _ = _factor_bank(issm, orc, rng, d, k, dtype, cuda, dof)
+    tdt = torch.float32 if dtype == np.float32 else torch.float64
+    slots = torch.tensor(rng.integers(0, k, size=n).astype(np.int32), device=cuda)
+    normals = torch.tensor(rng.normal(size=n * d).astype(dtype), device=cuda)
+    rad = {}
+    if dof:
+        rad = dict(radial_normals=torch.tensor(rng.normal(size=n * 8).astype(dtype), device=cuda), rn_stride=8,
+                   radial_uniforms=torch.tensor(rng.random(size=n * 8).astype(dtype), device=cuda), ru_stride=8)
+    den = issm.ops.denominator(issm.native.DENOM_FULL, torch.zeros(k, dtype=tdt, device=cuda))
+    db.proposal_ids = torch.arange(1, k + 1, device=cuda)
+    want = issm.ops.mis_round(db, den, slots, normals, **rad)
+    drawn = issm.ops.draw(db, normals, n, slots=slots, **rad)
+    for _ in range(5):
+        buf = normals.clone().view(n, d)
+        got = issm.ops.mis_round(db, den, slots, buf, samples=buf, **rad)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    buf = normals.clone().view(n, d)
+    assert torch.equal(issm.ops.draw(db, buf, n, slots=slots, out=buf, **rad), drawn)
