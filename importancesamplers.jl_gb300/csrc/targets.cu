@@ -200,6 +200,76 @@ __global__ void __launch_bounds__(256) target_regression_kernel(issm_target t, c
             if (ty * RS + i < rows) out[s0 + ty * RS + i] = constant + scale * acc[i].value() + prior_scale * bb[i];
 }
 
+// Few samples: a warp per sample, four observations per lane in flight, X straight
+// from global memory (coalesced; a CTA's four warps share its lines). The tiles above
+// put 16 samples on an SM, whose FP64 pipe bounds them: at 1,000 samples x 500
+// observations, d = 33, Gaussian, they take 88 us, this 49.
+constexpr int kRegRows = 4;  // warps, one per sub-partition
+constexpr int kRegFew = 32;  // samples per SM below which FP64 takes them
+template <typename T, bool LOGISTIC>
+__global__ void __launch_bounds__(32 * kRegRows) target_regression_rows_kernel(issm_target t, const T *__restrict__ x,
+                                                                              int64_t n, T constant, T scale,
+                                                                              T prior_scale, T *__restrict__ out) {
+    constexpr int kAhead = 4;  // coordinates whose loads are in flight together
+    const int d = t.dim, nobs = t.count, lane = threadIdx.x & 31;
+    const int64_t i = (int64_t)blockIdx.x * kRegRows + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const T *X = (const T *)t.a, *y = (const T *)t.b, *b = x + i * d;
+    T acc = T(0), prod = T(0), bb = T(0);
+    for (int c = lane; c < d; c += 32) bb += b[c] * b[c];
+    int steps = 0;
+    for (int o0 = lane; o0 < nobs; o0 += 128) {
+        T eta[4] = {T(0), T(0), T(0), T(0)};
+        const T *xo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xo[j] = X + min(o0 + 32 * j, nobs - 1);
+        int c = 0;
+#pragma unroll 1
+        for (; c + kAhead <= d; c += kAhead) {
+            T v[kAhead], xv[kAhead][4];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                v[u] = b[c + u];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) xv[u][j] = xo[j][(size_t)(c + u) * nobs];
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) eta[j] += xv[u][j] * v[u];
+        }
+#pragma unroll 1
+        for (; c < d; ++c) {
+            const T v = b[c];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) eta[j] += xo[j][(size_t)c * nobs] * v;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (o0 + 32 * j >= nobs) continue;
+            const T yv = y[o0 + 32 * j], e = eta[j];
+            if constexpr (LOGISTIC) {
+                const T f = dexp(-fabs(e));
+                prod += prod * f + f;
+                acc += yv * e - (e > T(0) ? e : isnan(e) ? e : T(0));
+            } else {
+                const T r = yv - e;
+                acc += r * r;
+            }
+        }
+        if (LOGISTIC && ++steps % kRegFlush == 0) {
+            acc -= dlog1p(prod);
+            prod = T(0);
+        }
+    }
+    if (LOGISTIC) acc -= dlog1p(prod);
+    for (int off = 16; off > 0; off >>= 1) {
+        acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        bb += __shfl_xor_sync(0xffffffffu, bb, off);
+    }
+    if (lane == 0) out[i] = constant + scale * acc + prior_scale * bb;
+}
+
 template <typename T, int RS>
 static int launch_regression(const issm_target *t, const T *x, int64_t n, T *out, cudaStream_t stream) {
     const double pv = (double)(T)t->p1, sg = (double)(T)t->p0;
@@ -209,6 +279,14 @@ static int launch_regression(const issm_target *t, const T *x, int64_t n, T *out
     const double scale = logistic ? 1.0 : -1.0 / (2.0 * sg * sg);
     const int dim_tile = min(t->dim, kRegDim);
     const size_t smem = sizeof(T) * (size_t)dim_tile * (16 * RS + 16 / sizeof(T) + kRegObs);
+    if constexpr (sizeof(T) == 8 && RS == 1)
+        if (n < kRegFew * (int64_t)device_sms()) {
+            const unsigned ctas = (unsigned)((n + kRegRows - 1) / kRegRows);
+            auto rows = logistic ? target_regression_rows_kernel<T, true> : target_regression_rows_kernel<T, false>;
+            rows<<<ctas, 32 * kRegRows, 0, stream>>>(*t, x, n, (T)constant, (T)scale, (T)(-1.0 / (2.0 * pv)), out);
+            note_launch();
+            return (int)cudaGetLastError();
+        }
     auto kern = target_regression_kernel<T, RS>;
     if (smem > 48 * 1024) {
         const int e = allow_dynamic_smem((const void *)kern);
