@@ -359,11 +359,13 @@ __global__ void __launch_bounds__(256) form_summary_kernel(const T *__restrict__
 }
 
 // CTAs of a summary: 16 weights per thread; FP64 weights take an FP64
-// exponential each in a serial chain, so two (57 us at n = 100,003 with 16).
+// exponential each in a serial chain, so two (57 us at n = 100,003 with 16) until
+// every SM has two CTAs: beyond, the last CTA's merge of more partials costs more
+// than the shorter chains save (129 us at n = 1,000,000 with eight, 112 with two).
 static int summary_blocks(int64_t n, int dtype) {
-    const int64_t per = 256 * (dtype == ISSM_F32 ? 16 : 2);
+    const int64_t per = 256 * (dtype == ISSM_F32 ? 16 : 2), cap = kSMs * (dtype == ISSM_F32 ? 8 : 2);
     int64_t b = (n + per - 1) / per;
-    if (b > kSMs * 8) b = kSMs * 8;
+    if (b > cap) b = cap;
     return b < 1 ? 1 : (int)b;
 }
 
