@@ -80,13 +80,15 @@ __global__ void __launch_bounds__(kMomThreads) mean_partial_kernel(const T *__re
             for (int r = r0; r < cnt; r += R) acc += wt[r] * (xp[r * d] - c0);
         }
     }
+    // the rows' sums in a fixed tree (256 of them one after the other took 15 us at d = 1)
     red[tid] = own ? (double)acc : 0.0;
-    __syncthreads();
-    if (tid < d) {
-        double s = 0.0;
-        for (int r = 0; r < R; ++r) s += red[r * d + tid];
-        partial[(size_t)blockIdx.x * d + tid] = s;
+    int half = 1;
+    while (half < R) half <<= 1;
+    for (half >>= 1; half > 0; half >>= 1) {
+        __syncthreads();
+        if (r0 < half && r0 + half < R) red[tid] += red[tid + half * d];
     }
+    if (tid < d) partial[(size_t)blockIdx.x * d + tid] = red[tid];
 }
 
 // Pass 2: sums of w z z^T, z = x - (mean rounded to T), over the lower
@@ -171,13 +173,15 @@ __global__ void __launch_bounds__(kCovThreads, 2) cov_partial_kernel(const T *__
     // the G sample lanes of a tile (adjacent lanes of one warp), then the H groups in order
     const int entries = tiles * R * R;
     double *red = reinterpret_cast<double *>(smem_raw);
+    const bool busy = (tid & ~31) < H * tiles * G;  // the other warps only staged samples
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             T v = acc[i][j];
-            for (int off = G >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (busy)
+                for (int off = G >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
             if (g == 0 && h < H) red[h * entries + tile * (R * R) + i * R + j] = (double)v;
         }
     __syncthreads();
@@ -239,10 +243,12 @@ template <typename T, int R>
 static int moments_t(const T *x, int d, int64_t n, const T *lw, const double *summary, const double *shift,
                      double *mean, double *cov, double *partial, cudaStream_t stream) {
     const int blocks = moment_blocks(n), tiles = cov_tiles(d, R);
+    // two samples at least for each of the H G lanes of a tile, whose sums are merged
+    // afterwards, and no more lanes than a step's samples
     int G = 32;
-    while (G > 1 && tiles * G > kCovThreads) G >>= 1;
-    const int H = max(1, kCovThreads / (tiles * G));  // > 1 for few tiles only (d <= 8)
-    const int threads = (H * tiles * G + 31) / 32 * 32;
+    while (G > 1 && (tiles * G > kCovThreads || n < 2 * G)) G >>= 1;
+    const int H = (int)max((int64_t)1, min((int64_t)(kCovThreads / (tiles * G)), min(n / 2, (int64_t)kMomTile) / G));
+    const int threads = max(128, (H * tiles * G + 31) / 32 * 32);
     constexpr int V = 16 / sizeof(T);
     int LD = (d + R - 1) / R * R;
     if (LD / V % 2 == 0) LD += V;  // an odd number of 16-byte groups per row
