@@ -58,6 +58,8 @@ template <typename T> struct MixParams {
     int mode;
     int first_slot, last_slot;
     int chunk, resident;   // components staged at a time; whether that is all of them, once per CTA
+    int whole;             // resident, and all of the bank
+    int nslots, nchunks;   // components evaluated; their chunks
     int ksplit;            // thread groups of a CTA that share its samples and split the components
     int prefetch;          // two sample tiles: the next one loads while one is evaluated
 };
@@ -480,6 +482,7 @@ __device__ __forceinline__ bool draw_row(const MixParams<T> &p, int slot, const 
                     for (int j = 0; j < 4; ++j) acc[j] += col[j] * z;
                 }
             } else {
+#pragma unroll 4
                 for (int q = 0; q < r0; ++q) {
                     const T z = in[q] * m;
 #pragma unroll
@@ -637,7 +640,7 @@ template <typename T, int D, bool FACTOR> __host__ __device__ constexpr bool sim
     return FACTOR && sizeof(T) == 4 && D <= 16;
 }
 
-// Mixture densities, static-MIS rounds, appends and draws. CTAs of 128 threads
+// Mixture densities, static-MIS rounds and appends. CTAs of 128 threads
 // walk tiles of samples; the bank is staged in shared memory, whole and once
 // per CTA when it fits (`resident`), else in double-buffered chunks prefetched
 // with asynchronous copies while the previous chunk is evaluated. Each thread
@@ -654,8 +657,8 @@ template <typename T, int D, bool FACTOR> __host__ __device__ constexpr bool sim
 template <typename T, int D, bool FACTOR, int S, int MINB>
 __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixParams<T> p) {
     using Ly = Layout<T, D, FACTOR>;
-    constexpr bool XREG = FACTOR && sizeof(T) == 4 && D <= 32;  // beyond, x and v together exceed the registers
     constexpr bool DIRECT = simt_direct<T, D, FACTOR>();
+    constexpr bool XREG = FACTOR && sizeof(T) == 4 && D <= 32;  // beyond, x and v together exceed the registers
     constexpr int LX = D + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *comps = reinterpret_cast<T *>(smem_raw);
@@ -666,8 +669,7 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
     T *drawn_tile = mult + kSimtThreads;         // and the drawn samples
     __shared__ int s_bad[kSimtThreads], s_lo, s_hi;
     const int grp = tid / GT, si = tid - grp * GT;
-    const int nslots = p.mode == kModeDraw ? 0 : p.last_slot - p.first_slot + 1;
-    const int nchunks = nslots > 0 ? (nslots + p.chunk - 1) / p.chunk : 0;
+    const int nslots = p.nslots, nchunks = p.nchunks;
     const int64_t ntiles = (p.n + TR - 1) / TR;
     const int my_tiles = (int)((ntiles - (int64_t)blockIdx.x + gridDim.x - 1) / gridDim.x);
     const bool only_own = p.den_kind == ISSM_DENOM_GENERATING;  // a tile needs its own samples' slots only
@@ -677,10 +679,9 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                                     min(p.chunk, nslots - k0));
     };
     // a draw's component: staged where the whole bank is, else null (a prefix may stop
-    // before a drawn slot, a plain draw stages none)
-    const bool whole = p.resident && nslots == p.k;
-    auto staged = [&](int slot) -> const T * { return whole ? comps + (size_t)slot * Ly::kStride : nullptr; };
-    const bool drawn = p.mode == kModeRound || p.mode == kModeDraw;
+    // before a drawn slot)
+    auto staged = [&](int slot) -> const T * { return p.whole ? comps + (size_t)slot * Ly::kStride : nullptr; };
+    const bool drawn = p.mode == kModeRound;
     const T *rows_in = drawn ? p.normals : p.x;
     auto tile_row = [&](int it) -> int64_t { return ((int64_t)blockIdx.x + (int64_t)it * gridDim.x) * TR; };
     auto request_rows = [&](int it) {
@@ -699,8 +700,8 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
     }
     const bool vec = DIRECT && d % Ly::V == 0 &&
                      ((reinterpret_cast<uintptr_t>(rows_in) | reinterpret_cast<uintptr_t>(p.samples_out)) & 15) == 0;
-    if (nslots > 0 && (p.resident || !only_own)) request(0, 0);
-    if (p.resident && nslots > 0) {
+    if (p.resident || !only_own) request(0, 0);
+    if (p.resident) {
         tc::cp_async_wait_all();
         __syncthreads();
         stage_finish<T, D, FACTOR>(comps, d, nslots);
@@ -751,7 +752,6 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                 __syncthreads();  // every group has its normals: the samples may take their place
                 if (grp == 0) put(0);
             }
-            if (p.mode == kModeDraw) continue;
             if (drawn && KS > 1) __syncthreads();  // the slow path reads the stored samples
         } else if (drawn) {
             if (KS == 1) {
@@ -787,7 +787,6 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                     record_failure(p.failures, p.index_base + row0 + si + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
             }
             if (p.samples_out) move_tile<T, LX, false>(xs, p.samples_out + (size_t)row0 * d, rows, d);
-            if (p.mode == kModeDraw) continue;
             __syncthreads();  // the slow path reads the stored samples
         }
         const T *xt = xs + (size_t)si * LX;
@@ -953,6 +952,66 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
             if (p.out_generating) p.out_generating[i] = gen_lq[s];
         }
     }
+}
+
+// Draws from given slots: a thread per sample, its row in registers, the components
+// from global memory (L1: the bank is small against the samples). Longer rows pass
+// through a shared tile, so that they are read and written whole lines at a time (FP32,
+// 100,000 x 64: 142 -> 112 us), except in FP64 beyond 32 coordinates, whose tile
+// leaves too few warps (d = 33, up to 10,000 samples: 47 -> 58). In the kernel above,
+// without registers to unroll into, FP64 draws of 100,000 x 33 took 268 us, here 172.
+template <typename T, int D> constexpr bool draw_slots_tile() { return D > 4 && D * sizeof(T) <= 256; }
+template <typename T, int D, bool FACTOR>
+__global__ void __launch_bounds__(kSimtThreads) draw_slots_kernel(MixParams<T> p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool TILE = draw_slots_tile<T, D>();
+    constexpr int LX = D + 1;
+    const int d = p.d;
+    const int64_t row0 = (int64_t)blockIdx.x * kSimtThreads, i = row0 + threadIdx.x;
+    const int rows = (int)min((int64_t)kSimtThreads, p.n - row0);
+    T *tile = reinterpret_cast<T *>(smem_raw);
+    if (TILE) {
+        move_tile<T, LX, true>(tile, const_cast<T *>(p.normals + (size_t)row0 * d), rows, d);
+        __syncthreads();
+    }
+    if (i < p.n) {
+        const int slot = p.slots ? p.slots[i] : p.fixed_slot;
+        const T m = draw_multiplier(p, i, slot);
+        const T *mu = p.loc + (size_t)slot * d, *in = TILE ? tile + threadIdx.x * LX : p.normals + (size_t)i * d;
+        T *out = TILE ? tile + threadIdx.x * LX : p.samples_out + (size_t)i * d;
+        T z[D];
+#pragma unroll
+        for (int c = 0; c < D; ++c) z[c] = c < d ? in[c] * m : T(0);
+        const T *L = p.scales + (size_t)slot * (p.scale_kind == ISSM_SCALE_SPHERICAL ? 1 : FACTOR ? d * d : d);
+        bool valid = true;
+#pragma unroll
+        for (int r = 0; r < D; ++r) {
+            if (r >= d) continue;
+            T v = mu[r];
+            if constexpr (FACTOR) {
+#pragma unroll
+                for (int c = 0; c <= r; ++c) v += L[r + (size_t)c * d] * z[c];
+            } else {
+                v += L[p.scale_kind == ISSM_SCALE_SPHERICAL ? 0 : r] * z[r];
+            }
+            out[r] = v;
+            valid &= (bool)isfinite(v);
+        }
+        if (!valid) record_failure(p.failures, p.index_base + i + 1, 0, ISSM_REASON_GENERATED_NONFINITE);
+    }
+    if (TILE) {
+        __syncthreads();
+        move_tile<T, LX, false>(tile, p.samples_out + (size_t)row0 * d, rows, d);
+    }
+}
+
+template <typename T, int D, bool FACTOR> static int launch_draw_slots(const MixParams<T> &p, cudaStream_t stream) {
+    if (p.n < 1) return 0;
+    auto kern = draw_slots_kernel<T, D, FACTOR>;
+    const size_t smem = draw_slots_tile<T, D>() ? (size_t)kSimtThreads * (D + 1) * sizeof(T) : 0;  // 34 KB at most
+    kern<<<(unsigned)((p.n + kSimtThreads - 1) / kSimtThreads), kSimtThreads, smem, stream>>>(p);
+    note_launch();
+    return (int)cudaGetLastError();
 }
 
 // Fixed-slot draws from one factor component, x = mu + L (m z) with the
@@ -1162,7 +1221,7 @@ template <typename T, int D, bool FACTOR, int S, int MINB>
 static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     using Ly = Layout<T, D, FACTOR>;
     if (p.n < 1) return 0;
-    const int nslots = p.mode == kModeDraw ? 0 : p.last_slot - p.first_slot + 1;
+    const int nslots = p.last_slot - p.first_slot + 1;
     const int sms = device_sms();
     auto tiles_of = [&](int ks) { return (p.n + kSimtThreads / ks * S - 1) / (kSimtThreads / ks * S); };
     // Components are split over thread groups while there are fewer than four
@@ -1184,10 +1243,13 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
         --want;
     const size_t budget = kSimtSmem / want - 1024 - fixed;
     p.resident = nslots * per <= budget;
+    p.whole = p.resident && nslots == p.k;
     // A second tile where it costs no CTA of the bank's: with few components the
     // tile's loads are most of a CTA's time.
     p.prefetch = p.resident && tiles > (int64_t)sms * want && nslots * per + rows_bytes <= budget;
     p.chunk = p.resident ? nslots : max(1, (int)(budget / 2 / per));
+    p.nslots = nslots;
+    p.nchunks = (nslots + p.chunk - 1) / p.chunk;
     const size_t smem = fixed + (p.prefetch ? rows_bytes : 0) + (p.resident ? 1 : 2) * (size_t)p.chunk * per;
     auto kern = mixture_simt_kernel<T, D, FACTOR, S, MINB>;
     if (smem > 46 * 1024) {  // the limit without opting in, less the static part
@@ -1239,9 +1301,19 @@ template <typename T> int dispatch_simt(const MixParams<T> &p0, cudaStream_t str
     // with one generating slot for every sample only that component counts
     if (p.mode == kModeDenominator && p.den_kind == ISSM_DENOM_GENERATING && p.slots == nullptr)
         p.first_slot = p.last_slot = p.fixed_slot;
+    if (p.mode == kModeDraw && (p.scale_kind != ISSM_SCALE_FACTOR || p.slots != nullptr)) {
+        const bool factor = p.scale_kind == ISSM_SCALE_FACTOR;
+#define ISSM_DRAW(DD) \
+    if (d <= DD) return factor ? launch_draw_slots<T, DD, true>(p, stream) : launch_draw_slots<T, DD, false>(p, stream);
+        ISSM_DRAW(4)
+        ISSM_DRAW(16)
+        ISSM_DRAW(32)
+        ISSM_DRAW(64)
+#undef ISSM_DRAW
+    }
     if (p.scale_kind != ISSM_SCALE_FACTOR)
         return d <= 8 ? launch_simt<T, 8, false, 1, 4>(p, stream) : launch_simt<T, 64, false, 1, 2>(p, stream);
-    if (p.mode == kModeDraw && p.slots == nullptr && p.samples_out != nullptr) {
+    if (p.mode == kModeDraw) {
         if (d <= 4) return launch_draw_fixed<T, 4>(p, stream);
         if (d <= 16) return launch_draw_fixed<T, 16>(p, stream);
         if (d <= 32) return launch_draw_fixed<T, 32>(p, stream);

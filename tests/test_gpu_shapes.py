@@ -672,3 +672,71 @@ def test_round_in_place(issm, orc, cuda, dtype, n, d, k, dof):
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     buf = normals.clone().view(n, d)
     assert torch.equal(issm.ops.draw(db, buf, n, slots=slots, out=buf, **rad), drawn)
+
+
+# A coordinate of a draw is a chain of at most d roundings of its terms and one of the mean:
+# (d + 2) eps of the sum of their sizes. Densities as in test_simt_density_shapes.
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("scale", ["factor", "diagonal", "spherical"])
+@pytest.mark.parametrize("n,d,k,dof", [(1, 1, 1, None), (127, 4, 3, None), (129, 5, 9, 5.0), (300, 8, 5, None),
+                                       (1000, 9, 33, None), (257, 16, 20, 4.0), (500, 17, 3, None), (129, 32, 7, None),
+                                       (260, 33, 4, 3.0), (128, 64, 2, None), (90_001, 3, 2, None), (90_001, 13, 5, None)])
+def test_simt_scale_kinds(issm, orc, cuda, dtype, scale, n, d, k, dof):
+    """Draws from given slots, rounds, densities and appends of every scale kind at
+    the edges of the padded dimensions."""
+    rng = np.random.default_rng(7 * d + k)
+    loc = rng.normal(size=(k, d)).astype(dtype)
+    if scale == "factor":
+        A = rng.normal(size=(k, d, d))
+        sc = np.linalg.cholesky(A @ A.transpose(0, 2, 1) / d + 0.5 * np.eye(d)).astype(dtype)
+        dense = sc.astype(np.float64)
+        make = issm.FactorGaussian if dof is None else lambda m, s: issm.FactorStudentT(dtype(dof), m, s)
+    elif scale == "diagonal":
+        sc = (0.5 + rng.random((k, d))).astype(dtype)
+        dense = sc[:, :, None].astype(np.float64) * np.eye(d)
+        make = issm.DiagonalGaussian if dof is None else lambda m, s: issm.DiagonalStudentT(dtype(dof), m, s)
+    else:
+        sc = (0.5 + rng.random(k)).astype(dtype)
+        dense = sc[:, None, None].astype(np.float64) * np.eye(d)
+        make = issm.SphericalGaussian if dof is None else lambda m, s: issm.SphericalStudentT(dtype(dof), m, s)
+    db = issm.pack_proposals([make(m, s) for m, s in zip(loc, sc)], cuda)
+    ob = orc.BankView(d, orc.GAUSSIAN if dof is None else orc.STUDENT_T,
+                      {"factor": orc.SCALE_FACTOR, "diagonal": orc.SCALE_DIAGONAL, "spherical": orc.SCALE_SPHERICAL}[scale],
+                      db.locations.double().cpu().numpy(), db.scales.double().cpu().numpy(),
+                      db.lognormalizers.double().cpu().numpy(), None if dof is None else db.dofs.double().cpu().numpy(),
+                      None if db.range_risk is None else db.range_risk.cpu().numpy())
+    tdt = torch.float32 if dtype == np.float32 else torch.float64
+    slots = rng.integers(0, k, size=n).astype(np.int32)
+    ts = torch.tensor(slots, device=cuda)
+    z = rng.normal(size=(n, d)).astype(dtype)
+    rad, mult = {}, np.ones((n, 1))
+    if dof:
+        # uniforms of zero accept the first normal that gives a positive cube: the multiplier is smooth in it
+        rn, ru = 0.2 * rng.normal(size=(n, 8)), np.zeros((n, 8))
+        rad = dict(radial_normals=torch.tensor(rn.reshape(-1).astype(dtype), device=cuda), rn_stride=8,
+                   radial_uniforms=torch.tensor(ru.reshape(-1).astype(dtype), device=cuda), ru_stride=8)
+        off = np.float64(dof) / 2 - 1 / 3
+        mult = np.sqrt(dof / (2 * off * (1 + rn[:, :1].astype(dtype).astype(np.float64) / (3 * np.sqrt(off))) ** 3))
+    x = issm.ops.draw(db, torch.tensor(z.reshape(-1), device=cuda), n, slots=ts, **rad)
+    zm = z.astype(np.float64) * mult
+    want = loc[slots].astype(np.float64) + np.einsum("irc,ic->ir", dense[slots], zm)
+    size = np.abs(loc[slots]).astype(np.float64) + np.einsum("irc,ic->ir", np.abs(dense[slots]), np.abs(zm))
+    # a multiplier holds at most ten roundings
+    assert np.all(np.abs(x.double().cpu().numpy() - want) <= (d + (14 if dof else 2)) * float(np.finfo(dtype).eps) * size)
+    coef = np.log(rng.dirichlet(np.ones(k))).astype(dtype)
+    tc = torch.tensor(coef, device=cuda)
+    db.proposal_ids = torch.arange(1, k + 1, device=cuda)
+    tol = 1e-12 if dtype == np.float64 else 2e-5
+    xs = x.double().cpu().numpy().reshape(-1)
+    for kind, okind in ((issm.native.DENOM_FULL, orc.DENOM_FULL), (issm.native.DENOM_GENERATING, orc.DENOM_GENERATING)):
+        den = issm.ops.denominator(kind, tc)
+        rx, lw, _ = issm.ops.mis_round(db, den, ts, torch.tensor(z.reshape(-1), device=cuda), **rad)
+        got = issm.ops.mixture_logdensity(db, den, x, slots=ts)
+        exp, _, _ = orc.mixture_logdensity(ob, xs, okind, coef.astype(np.float64), slots=slots)
+        assert torch.equal(rx, x) and torch.equal(lw, -got)
+        assert np.all(np.abs(got.double().cpu().numpy() - exp) <= tol * np.maximum(1.0, np.abs(exp)))
+    lognum = torch.tensor(exp.astype(dtype), device=cuda)
+    issm.ops.amis_append(db.ref(), k - 1, tc, x, lognum)
+    lq, _, _ = orc.mixture_logdensity(ob, xs, orc.DENOM_GENERATING, slots=None, fixed_slot=k - 1)
+    expa = np.logaddexp(exp.astype(dtype).astype(np.float64), coef[-1].astype(np.float64) + lq)
+    assert np.all(np.abs(lognum.double().cpu().numpy() - expa) <= tol * np.maximum(1.0, np.abs(expa)))
