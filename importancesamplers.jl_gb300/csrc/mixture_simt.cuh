@@ -550,12 +550,24 @@ template <typename T, int D> __device__ __forceinline__ void store_row(T *g, int
 }
 
 // draw_row in registers: x holds the normals, then the sample
-template <typename T, int D>
+template <typename T, int D, bool FACTOR>
 __device__ __forceinline__ bool draw_registers(const MixParams<T> &p, int slot, const T *c, T m, T (&x)[D]) {
-    using Ly = Layout<T, D, true>;
+    using Ly = Layout<T, D, FACTOR>;
     constexpr int V = Ly::V;
     const int d = p.d;
     const T *mu = c ? c + Ly::kMu : p.loc + (size_t)slot * d;
+    if constexpr (!FACTOR) {
+        const bool one = p.scale_kind == ISSM_SCALE_SPHERICAL;
+        const T *sc = c ? c + Ly::kBody : one ? p.scales + slot : p.scales + (size_t)slot * d;
+        bool valid = true;
+#pragma unroll
+        for (int r = 0; r < D; ++r)
+            if (r < d) {
+                x[r] = mu[r] + sc[c || !one ? r : 0] * (x[r] * m);
+                valid &= (bool)isfinite(x[r]);
+            }
+        return valid;
+    }
     const T *L = p.scales + (size_t)slot * d * d;
     T y[D];
 #pragma unroll
@@ -636,9 +648,7 @@ template <typename T, int LX> __device__ __forceinline__ void request_tile(T *ti
 }
 
 // rows go between global memory and registers, without a tile
-template <typename T, int D, bool FACTOR> __host__ __device__ constexpr bool simt_direct() {
-    return FACTOR && sizeof(T) == 4 && D <= 16;
-}
+template <typename T, int D> __host__ __device__ constexpr bool simt_direct() { return sizeof(T) == 4 && D <= 16; }
 
 // Mixture densities, static-MIS rounds and appends. CTAs of 128 threads
 // walk tiles of samples; the bank is staged in shared memory, whole and once
@@ -654,11 +664,10 @@ template <typename T, int D, bool FACTOR> __host__ __device__ constexpr bool sim
 // samples and the bank restaged element by element by each took 11.9 ms for a
 // static-MIS call of 4,194,304 samples, d = 16, 64 components (now 3.5 ms), and
 // 2.38 ms for a population round of 16,384 samples, d = 32, 256 components (1.30).
-template <typename T, int D, bool FACTOR, int S, int MINB>
+template <typename T, int D, bool FACTOR, int S, int MINB, bool DIRECT>
 __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixParams<T> p) {
     using Ly = Layout<T, D, FACTOR>;
-    constexpr bool DIRECT = simt_direct<T, D, FACTOR>();
-    constexpr bool XREG = FACTOR && sizeof(T) == 4 && D <= 32;  // beyond, x and v together exceed the registers
+    constexpr bool XREG = DIRECT || (FACTOR && sizeof(T) == 4 && D <= 32);  // beyond, x and v together exceed the registers
     constexpr int LX = D + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *comps = reinterpret_cast<T *>(smem_raw);
@@ -745,7 +754,7 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
                 const int64_t i = row0 + si + s * GT;
                 load_row<T, D>(rows_in + (size_t)(ok[s] ? i : 0) * d, d, vec, x[s]);
                 if (drawn && ok[s])
-                    ok[s] = draw_registers<T, D>(p, gen[s], staged(gen[s]), draw_multiplier(p, i, gen[s], grp == 0), x[s]);
+                    ok[s] = draw_registers<T, D, FACTOR>(p, gen[s], staged(gen[s]), draw_multiplier(p, i, gen[s], grp == 0), x[s]);
                 if (drawn && KS == 1) put(s);
             }
             if (S == 1 && drawn && KS > 1) {
@@ -857,11 +866,18 @@ __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixPar
 #pragma unroll
                     for (int s = 0; s < S; ++s) {
                         r2[s] = T(0);
-                        for (int r = 0; r < d; ++r) {
-                            const T dv = xt[s * GT * LX + r] - c[Ly::kMu + r];
+                        auto add = [&](T xr, int r) {
+                            const T dv = xr - c[Ly::kMu + r];
                             const T v = sizeof(T) == 4 ? dv * c[Ly::kInv + r]
                                                        : quotient(dv, c[Ly::kBody + r], c[Ly::kInv + r]);
                             r2[s] += v * v;
+                        };
+                        if constexpr (XREG) {
+#pragma unroll
+                            for (int r = 0; r < D; ++r)
+                                if (r < d) add(x[s][r], r);
+                        } else {
+                            for (int r = 0; r < d; ++r) add(xt[s * GT * LX + r], r);
                         }
                     }
                 }
@@ -1217,7 +1233,7 @@ template <typename T, int D> static int launch_draw_fixed(const MixParams<T> &p,
 
 constexpr size_t kSimtSmem = 227 * 1024;  // shared memory of an SM that CTAs can take (1 KB each reserved)
 
-template <typename T, int D, bool FACTOR, int S, int MINB>
+template <typename T, int D, bool FACTOR, int S, int MINB, bool DIRECT = simt_direct<T, D>()>
 static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     using Ly = Layout<T, D, FACTOR>;
     if (p.n < 1) return 0;
@@ -1234,7 +1250,7 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     p.ksplit = ks;
     const int64_t tiles = tiles_of(ks);
     const size_t per = (size_t)Ly::kStride * sizeof(T);
-    const size_t rows_bytes = simt_direct<T, D, FACTOR>() ? 0 : (size_t)(kSimtThreads / ks) * S * (D + 1) * sizeof(T);
+    const size_t rows_bytes = DIRECT ? 0 : (size_t)(kSimtThreads / ks) * S * (D + 1) * sizeof(T);
     const size_t fixed = rows_bytes + (ks > 1 ? (size_t)kSimtThreads * 5 * sizeof(T) + rows_bytes : 0);
     // the bank's share of shared memory with as many CTAs on an SM as the
     // registers allow, or as there are; one fewer where the bank then stays
@@ -1251,7 +1267,7 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     p.nslots = nslots;
     p.nchunks = (nslots + p.chunk - 1) / p.chunk;
     const size_t smem = fixed + (p.prefetch ? rows_bytes : 0) + (p.resident ? 1 : 2) * (size_t)p.chunk * per;
-    auto kern = mixture_simt_kernel<T, D, FACTOR, S, MINB>;
+    auto kern = mixture_simt_kernel<T, D, FACTOR, S, MINB, DIRECT>;
     if (smem > 46 * 1024) {  // the limit without opting in, less the static part
         const int e = allow_dynamic_smem((const void *)kern);
         if (e) return e;
@@ -1311,8 +1327,13 @@ template <typename T> int dispatch_simt(const MixParams<T> &p0, cudaStream_t str
         ISSM_DRAW(64)
 #undef ISSM_DRAW
     }
-    if (p.scale_kind != ISSM_SCALE_FACTOR)
-        return d <= 8 ? launch_simt<T, 8, false, 1, 4>(p, stream) : launch_simt<T, 64, false, 1, 2>(p, stream);
+    if (p.scale_kind != ISSM_SCALE_FACTOR) {
+        constexpr int kMinB = sizeof(T) == 4 ? 8 : 4;
+        if (d <= 4) return launch_simt<T, 4, false, 1, kMinB>(p, stream);
+        if (d <= 8) return launch_simt<T, 8, false, 1, kMinB>(p, stream);
+        if (d <= 16) return launch_simt<T, 16, false, 1, kMinB>(p, stream);
+        return launch_simt<T, 64, false, 1, 2>(p, stream);
+    }
     if (p.mode == kModeDraw) {
         if (d <= 4) return launch_draw_fixed<T, 4>(p, stream);
         if (d <= 16) return launch_draw_fixed<T, 16>(p, stream);
