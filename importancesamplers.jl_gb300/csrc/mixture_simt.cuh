@@ -346,7 +346,7 @@ __device__ __forceinline__ void factor_radius(const T *__restrict__ c, const T (
         for (int s = 0; s < S; ++s)
 #pragma unroll
             for (int j = 0; j < V; ++j) {
-                if constexpr (XREG) v[s][r0 + j] = x[s][r0 + j] - mu[j];
+                if constexpr (XREG) v[s][r0 + j] = !kSkip || r0 < d ? x[s][r0 + j] - mu[j] : T(0);
                 else v[s][r0 + j] = !kSkip || r0 < d ? xt[s * step + r0 + j] - mu[j] : T(0);
             }
     }
@@ -1241,12 +1241,15 @@ static int launch_simt(MixParams<T> p, cudaStream_t stream) {
     const int sms = device_sms();
     auto tiles_of = [&](int ks) { return (p.n + kSimtThreads / ks * S - 1) / (kSimtThreads / ks * S); };
     // Components are split over thread groups while there are fewer than four
-    // CTAs per SM (FP32), or than eight waves of them: FP64 runs at the pipe's
-    // rate from one warp per scheduler on, so finer tiles only even out the last
-    // wave. A generating-only denominator has one component per sample to split.
+    // CTAs per SM, FP64 from eight components per group on than eight waves of them:
+    // it runs at the pipe's rate from one warp per scheduler on, so finer tiles only
+    // even out the last wave, for the price of the merge's exponentials. A
+    // generating-only denominator has one component per sample to split.
     int ks = 1;
     if (S == 1 && nslots > 1 && p.den_kind != ISSM_DENOM_GENERATING)
-        while (ks < 4 && nslots >= 2 * ks && tiles_of(ks) < (int64_t)sms * min(MINB, 4) * (sizeof(T) == 8 ? 8 : 1)) ks *= 2;
+        while (ks < 4 && nslots >= 2 * ks &&
+               tiles_of(ks) < (int64_t)sms * min(MINB, 4) * (sizeof(T) == 8 && nslots >= 16 * ks ? 8 : 1))
+            ks *= 2;
     p.ksplit = ks;
     const int64_t tiles = tiles_of(ks);
     const size_t per = (size_t)Ly::kStride * sizeof(T);
@@ -1302,7 +1305,10 @@ template <typename T> static int dispatch_factor(const MixParams<T> &p, cudaStre
         if (d <= 48) return launch_simt<T, 48, true, 1, 3>(p, stream);
         return launch_simt<T, 64, true, 1, 3>(p, stream);
     } else {
-        if (d <= 4) return launch_simt<T, 4, true, 1, 4>(p, stream);
+        // short FP64 rows straight into registers, but not for draws, which thread groups share
+        if (d <= 4)
+            return p.mode == kModeDenominator || p.mode == kModeAppend ? launch_simt<T, 4, true, 1, 4, true>(p, stream)
+                                                                       : launch_simt<T, 4, true, 1, 4>(p, stream);
         if (d <= 8) return launch_simt<T, 8, true, 1, 4>(p, stream);
         if (d <= 16) return launch_simt<T, 16, true, 1, 4>(p, stream);
         if (d <= 32) return launch_simt<T, 32, true, 1, 4>(p, stream);
