@@ -1,6 +1,6 @@
 // tc_selftest.cu — a one-CTA tcgen05 GEMM, C[128 x n] = A[128 x k] B[n x k]^T,
-// used by the test suite to pin the descriptor encodings (tcgen05.cuh) that
-// every tensor-core kernel of this library relies on. Inputs are FP32 and are
+// used by the test suite to pin the descriptor encodings and the elected issue
+// (tcgen05.cuh) that every tensor-core kernel of this library relies on. Inputs are FP32 and are
 // rounded to bf16 or tf32 while staged into shared memory.
 #include "issm_device.cuh"
 #include "issm_internal.h"
@@ -48,8 +48,8 @@ __global__ void __launch_bounds__(128) tc_gemm_selftest_kernel(const float *__re
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tbase = tmem_base;
-    if (threadIdx.x == 0) {
+    const uint32_t tbase = tc::uniform(tmem_base);
+    if (tc::uniform_warp() == 0) {
         const uint32_t idesc = tc::instr_desc(kind, 128, n) | (layout >= 2 ? tc::kMajorMN : 0u);
         const int steps = k * eb / 32;
         for (int s = 0; s < steps; ++s) {
@@ -65,10 +65,10 @@ __global__ void __launch_bounds__(128) tc_gemm_selftest_kernel(const float *__re
                 da = tc::smem_desc(tc::smem_u32(sa) + s * 256, 128, kg * 128);
                 db = tc::smem_desc(tc::smem_u32(sb) + s * 256, 128, kg * 128);
             }
-            if (kind == tc::kBF16) tc::mma(tbase, da, db, idesc, s > 0);
-            else tc::mma_tf32(tbase, da, db, idesc, s > 0);
+            if (kind == tc::kBF16) tc::mma_elect(tbase, da, db, idesc, s > 0);
+            else tc::mma_tf32_elect(tbase, da, db, idesc, s > 0);
         }
-        tc::commit(&bar);
+        tc::commit_elect(&bar);
     }
     const bool ok = tc::mbar_wait(&bar, 0);
     if (!ok && threadIdx.x == 0) atomicExch(status, 1);
