@@ -173,17 +173,16 @@ __global__ void __launch_bounds__(kCovThreads, 2) cov_partial_kernel(const T *__
     // the G sample lanes of a tile (adjacent lanes of one warp), then the H groups in order
     const int entries = tiles * R * R;
     double *red = reinterpret_cast<double *>(smem_raw);
-    const bool busy = (tid & ~31) < H * tiles * G;  // the other warps only staged samples
     __syncthreads();
+    if ((tid & ~31) < H * tiles * G)  // the other warps only staged samples
 #pragma unroll
-    for (int i = 0; i < R; ++i)
+        for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int j = 0; j < R; ++j) {
-            T v = acc[i][j];
-            if (busy)
+            for (int j = 0; j < R; ++j) {
+                T v = acc[i][j];
                 for (int off = G >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-            if (g == 0 && h < H) red[h * entries + tile * (R * R) + i * R + j] = (double)v;
-        }
+                if (g == 0 && h < H) red[h * entries + tile * (R * R) + i * R + j] = (double)v;
+            }
     __syncthreads();
     for (int e = tid; e < entries; e += B) {
         double s = red[e];

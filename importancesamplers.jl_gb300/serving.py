@@ -201,8 +201,8 @@ def _cdiv(a, b):
 
 
 class _Prep:
-    """Host side of one grouped run, computed off the serving thread: the
-    target's exact mode-centred form from its sufficient statistics, the byte
+    """Host side of one grouped run, computed on the serving thread while the
+    device steps the admitted runs: the target's exact mode-centred form from its sufficient statistics, the byte
     layout of the run's single device allocation, and the bytes admission
     writes (zeroed failure words, the target's mode and factor, the history's
     slot 0)."""
