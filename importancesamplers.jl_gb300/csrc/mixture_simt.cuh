@@ -662,8 +662,10 @@ template <typename T, int D> __host__ __device__ constexpr bool simt_direct() { 
 // load costs about 2.4 clocks of an SM; two samples per load is where FMAs
 // overtake loads) or by the FP64 pipe. One thread per sample, one CTA per 128
 // samples and the bank restaged element by element by each took 11.9 ms for a
-// static-MIS call of 4,194,304 samples, d = 16, 64 components (now 3.5 ms), and
-// 2.38 ms for a population round of 16,384 samples, d = 32, 256 components (1.30).
+// static-MIS call of 4,194,304 samples, d = 16, 64 components (now 2.9 ms, 2.6 of
+// them this kernel: 263 issue slots per sample and component, 190 on the FMA pipe, 136
+// of those the substitution's), and 1.33 ms in the kernel for a population round of
+// 16,384 samples, d = 32, 256 components (0.25).
 template <typename T, int D, bool FACTOR, int S, int MINB, bool DIRECT>
 __global__ void __launch_bounds__(kSimtThreads, MINB) mixture_simt_kernel(MixParams<T> p) {
     using Ly = Layout<T, D, FACTOR>;

@@ -239,7 +239,8 @@ int issm_amis_append_ws(const issm_bank *history, int32_t slot,
  * logw_i = logtarget_i - logden_i when `logtargets` is non-NULL; with
  * logtargets == NULL the target is deferred (the reference's batch-target
  * path, src/batched_targets.jl:70-77) and logw_i = -logden_i, finished later
- * by issm_add_target_values. proposal_ids_out[i] = proposal_ids[slot] (or 0
+ * by issm_add_target_values. `samples` may be the array of `normals`, here and
+ * in issm_draw. proposal_ids_out[i] = proposal_ids[slot] (or 0
  * on failure). Replaces _mis_round_launch_kernel! (src/mis_execution.jl:674-720). */
 int issm_mis_round(const issm_bank *bank, const issm_denominator *den,
                    const int32_t *slots, const void *normals,
@@ -449,10 +450,11 @@ int issm_weighted_sum(const void *x, int32_t d, int64_t n, const void *logweight
  * component-wise weighted quantiles with the StatsBase generic-weight rule
  * (threshold p (W - w_first) + w_first over the value-sorted positive-weight
  * samples, linear interpolation between the neighbours), on the device with
- * no sort (a weighted radix select); out[q * d + c] for probability q and
- * coordinate c, in FP64 holding the sample type's value; NaN for a
- * coordinate with a NaN sample. probabilities: device FP64, each in [0, 1]
- * (the caller checks). The reference evaluates it on the host only. */
+ * no sort of the samples (value buckets, then key intervals);
+ * out[q * d + c] for probability q and coordinate c, in FP64 holding the
+ * sample type's value; NaN for a coordinate with a NaN sample.
+ * probabilities: device FP64, each in [0, 1] (the caller checks). The
+ * reference evaluates it on the host only. */
 size_t issm_weighted_quantile_workspace_bytes(int32_t d, int32_t nprob);
 int issm_weighted_quantile(const void *x, int32_t d, int64_t n, const void *logweights,
                            int32_t dtype, const double *summary,

@@ -740,3 +740,47 @@ def test_simt_scale_kinds(issm, orc, cuda, dtype, scale, n, d, k, dof):
     lq, _, _ = orc.mixture_logdensity(ob, xs, orc.DENOM_GENERATING, slots=None, fixed_slot=k - 1)
     expa = np.logaddexp(exp.astype(dtype).astype(np.float64), coef[-1].astype(np.float64) + lq)
     assert np.all(np.abs(lognum.double().cpu().numpy() - expa) <= tol * np.maximum(1.0, np.abs(expa)))
+
+
+@pytest.mark.parametrize("form", ["bf16", "tf32"])
+@pytest.mark.parametrize("d,k", [(64, 5), (33, 9), (16, 40)])
+def test_paired_tiles_around_one_per_sm(issm, cuda, form, d, k):
+    """As many tiles as SMs and one more, where a CTA begins to take two: the
+    rows' numbers do not change."""
+    rng = np.random.default_rng(d)
+    props = [issm.FactorGaussian(rng.normal(size=d).astype(np.float32),
+                                 (np.eye(d) + 0.1 * np.tril(rng.normal(size=(d, d)), -1)).astype(np.float32))
+             for _ in range(k)]
+    db = issm.pack_proposals(props, cuda)
+    db.attach_inverse_factors()
+    prec = issm.native.PREC_BF16 if form == "bf16" else issm.native.PREC_TF32
+    den = issm.ops.denominator(issm.native.DENOM_FULL, torch.zeros(k, device=cuda))
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    n = 128 * sms
+    x = torch.randn(2 * n + 3, d, device=cuda, generator=torch.Generator(device=cuda).manual_seed(2))
+    want = issm.ops.mixture_logdensity(db, den, x, precision=prec)
+    assert bool(torch.isfinite(want).all())
+    for m in (n - 127, n, n + 1):
+        assert torch.equal(issm.ops.mixture_logdensity(db, den, x[:m], precision=prec), want[:m])
+    issm.ops.check_tensor_core_errors(cuda)
+
+
+@pytest.mark.parametrize("kind", ["logistic", "linreg"])
+@pytest.mark.parametrize("d,nobs,n", [(1, 31, 5), (3, 129, 3), (4, 128, 4863), (6, 2100, 4864), (66, 33, 9)])
+def test_f64_regression_of_few_samples(issm, cuda, kind, d, nobs, n):
+    """A warp per sample and the line to the tiles, within the bounds of
+    test_simt_regression_shapes."""
+    test_simt_regression_shapes(issm, cuda, np.float64, kind, d, nobs, n)
+
+
+# Each exponential holds 1 ulp and its argument's rounding (16 eps at most here), each sum
+# n / (512 x 304) + 20 roundings: 64 eps of the sums covers both.
+@pytest.mark.parametrize("n", [1, 511, 513, 155_647, 155_649, 700_001])
+def test_f64_summary_grid(issm, cuda, n):
+    lw = torch.randn(n, device=cuda, dtype=torch.float64, generator=torch.Generator(device=cuda).manual_seed(n)) * 3.0
+    got = issm.ops.logweight_summary(lw).cpu().numpy()
+    l = lw.cpu().numpy()
+    e = np.exp(l - l.max())
+    assert got[0] == l.max()
+    assert abs(got[1] - e.sum()) <= 64 * 2.0**-52 * e.sum()
+    assert abs(got[2] - (e * e).sum()) <= 64 * 2.0**-52 * (e * e).sum()
